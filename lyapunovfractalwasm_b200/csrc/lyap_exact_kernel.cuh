@@ -35,10 +35,10 @@ static __device__ const lyap_logtab_entry g_lyap_logtab[LYAP_LOG_BINS] = {LYAP_L
 
 constexpr int kTabCopies = 8;
 constexpr size_t kTabSmemBytes = (size_t)LYAP_LOG_BINS * kTabCopies * sizeof(lyap_logtab_entry);  // 128 KB
-// Second shared table, indexed by the top 12 bits of the derivative (sign + exponent field e): {e*LN2HI (exact),
-// (e-1023)*LN2LO}.  It replaces an integer->double conversion and one fma per logarithm, and it carries the
-// irregular cases: entry 0 (zero or subnormal derivative) is -inf and entries >= 2047 (inf, NaN, sign bit) are NaN,
-// so such a step poisons the running sum and the chunk is redone step by step.
+// Second shared table, indexed by the top 12 bits of HALF the derivative (sign + exponent field e - 1, where e is the
+// derivative's own field): {e*LN2HI (exact), (e-1023)*LN2LO}.  It replaces an integer->double conversion and one fma per
+// logarithm, and it carries the irregular cases: entry 0 (zero or subnormal) is -inf and entries >= 2046 (a derivative
+// that is inf or NaN, sign bit) are NaN, so such a step poisons the running sum and the chunk is redone step by step.
 constexpr int kExpEntries = 4096;
 constexpr size_t kExpSmemBytes = (size_t)kExpEntries * sizeof(double2);                              // 64 KB
 constexpr size_t kExactSmemBytes = kTabSmemBytes + kExpSmemBytes;
@@ -93,6 +93,15 @@ __device__ __noinline__ bool careful_chunk(PixelState* ps, double rA, double rB,
     return dead;
 }
 
+// |r*(1-2x)| / 2 for r > 0, with the reference's rounding: 1 - 2x = 2*(0.5 - x), and a factor of two changes no rounding
+// (the smallest non-zero 0.5 - x is 2^-54, so nothing gets near the subnormals for ordinary r).  The subtraction reads one
+// register pair where fma(-2, x, 1) reads two, its second constant being one: the lambda kernel is bound by register reads
+// (a 64-bit pair a cycle and scheduler: two-operand fp64 instructions alone use them up, measured 1.98 cycles each, 2.96
+// with three distinct registers), and this one read fewer took 4096 x 2048 pixels of
+// "AABAB" 200 + 2000 from 16.11 to 15.73 ms.  What remains is the look-ups: two 16-byte loads a logarithm keep the SM's one
+// shared-memory data pipe busy for 32 of the 34 cycles that a scheduler now takes for a pixel and step.
+__device__ __forceinline__ double half_derivative(double r, double x) { return __dmul_rn(r, fabs(__dsub_rn(0.5, x))); }
+
 // Constants of the log core in constant memory: fp64 instructions take them as constant-bank
 // operands, which costs no instruction (64-bit immediates would each need two moves).
 struct LogConsts {
@@ -101,7 +110,7 @@ struct LogConsts {
 static __constant__ LogConsts c_logk = {LYAP_LOG_C2, LYAP_LOG_C3, LYAP_LOG_C4, LYAP_LN2HI, LYAP_LN2LO, LYAP_KLO_BIAS};
 static __constant__ int c_minus_2p20 = -(1 << 20);   // read as a constant-bank operand so the product below stays one multiply-add
 
-// lyap_log_core (lyap_math.h) for a positive normal d, written against the two shared-memory tables, which start
+// lyap_log_core (lyap_math.h) of 2*d for a positive normal d, written against the two shared-memory tables, which start
 // at the beginning of the dynamic shared memory: `lane_off` is the byte offset of this lane's copy inside a
 // mantissa-table entry group ((lane & 7) * 16; groups are kTabCopies*16 bytes apart), or'ed into the bin offset so
 // that the address is one logic operation plus a constant.  Same values in the same order as
@@ -165,8 +174,7 @@ __device__ __forceinline__ void fast_group(double (&x)[P], double (&lyap)[P], co
             double r = not_a ? rB[p] : rA[p];
             if (HAS_C) r = is_c ? rC : r;
             if (ACC) {
-                const double t = __fma_rn(-2.0, x[p], 1.0);      // == fl(1 - fl(2x)): 2x is exact
-                d[j][p] = __dmul_rn(r, fabs(t));                 // == |r*(1-2x)| for r > 0
+                d[j][p] = half_derivative(r, x[p]);
             }
             x[p] = __dmul_rn(__dmul_rn(r, x[p]), __dsub_rn(1.0, x[p]));
         }
@@ -198,8 +206,7 @@ __device__ __forceinline__ void fixed_group(double (&x)[P], double (&lyap)[P], c
         for (int p = 0; p < P; ++p) {
             const double r = code == 0 ? rA[p] : (code == 1 ? rB[p] : rC);
             if (ACC) {
-                const double t = __fma_rn(-2.0, x[p], 1.0);      // == fl(1 - fl(2x)): 2x is exact
-                d[j][p] = __dmul_rn(r, fabs(t));                 // == |r*(1-2x)| for r > 0
+                d[j][p] = half_derivative(r, x[p]);
             }
             x[p] = __dmul_rn(__dmul_rn(r, x[p]), __dsub_rn(1.0, x[p]));
         }
@@ -324,8 +331,8 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
     for (int e = threadIdx.x; e < kExpEntries; e += THREADS) {
         double2 v;
         if (e == 0) v = make_double2(__longlong_as_double(0xFFF0000000000000LL), 0.0);                       // zero / subnormal derivative
-        else if (e >= 2047) v = make_double2(__longlong_as_double(0x7FF8000000000000LL), 0.0);                // inf, NaN, or a set sign bit
-        else v = make_double2(__dmul_rn((double)e, LYAP_LN2HI), __fma_rn((double)e, LYAP_LN2LO, LYAP_KLO_BIAS));
+        else if (e >= 2046) v = make_double2(__longlong_as_double(0x7FF8000000000000LL), 0.0);                // inf, NaN, or a set sign bit
+        else v = make_double2(__dmul_rn((double)(e + 1), LYAP_LN2HI), __fma_rn((double)(e + 1), LYAP_LN2LO, LYAP_KLO_BIAS));
         exp_tab[e] = v;
     }
     __syncthreads();   // both tables are read across warps from the first logarithm on (at once when warmup == 0)
