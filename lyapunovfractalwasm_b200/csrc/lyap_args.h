@@ -15,6 +15,7 @@ struct LambdaArgs {
     double min_x, min_y, dx, dy, c_value;
     long long row_begin;   // global index of the first row of this launch
     long long n_pixels;    // rows * width
+    long long wide_tiles;  // exact kernel: warp-tiles of several pixels a thread, before the rest goes in tiles of one
     int width;
     int warmup, iterations;
     int acc_word0;

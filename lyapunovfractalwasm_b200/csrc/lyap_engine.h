@@ -24,7 +24,7 @@ cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out
 // (0 never, 1 once enough work with this sequence has been seen, 2 at once); kSpecUsePrebuilt allows the instances
 // compiled at build time (lyap_prebuilt.cu), which are tried first.
 constexpr int kSpecUsePrebuilt = 4;
-cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, int sm_count,
+cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, unsigned grid,
                                cudaStream_t st, int kind, int pixels_per_thread, int threads, size_t smem_bytes, int mode,
                                bool* launched);
 const char* jit_last_note();

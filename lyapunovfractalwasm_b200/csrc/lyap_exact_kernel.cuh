@@ -314,175 +314,97 @@ __host__ __device__ constexpr bool pats_use_c(unsigned long long pats) {
     return (pats & 0xAAAAAAAAAAAAAAAAull) != 0;
 }
 
-// Body shared by the library's generic kernel (KG == 0: patterns dispatched at run time) and by a specialised
-// instance (KG > 0: WU_PATS / ACC_PATS are the group patterns of the warm-up and accumulation regions).
-template <int P, int THREADS, bool HAS_C, int UNROLL, int KG, unsigned long long WU_PATS, unsigned long long ACC_PATS>
-__device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* __restrict__ out64, float* __restrict__ out32,
-                  unsigned long long* __restrict__ steps_out) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    lyap_logtab_entry* tab_all = reinterpret_cast<lyap_logtab_entry*>(smem_raw);
-    for (int e = threadIdx.x; e < LYAP_LOG_BINS * kTabCopies; e += THREADS) {
-        lyap_logtab_entry t = g_lyap_logtab[e / kTabCopies];
-        t.invc = __hiloint2double(__double2hiint(t.invc) + 0x3FF00000, __double2loint(t.invc));   // see log_fast
-        tab_all[e] = t;
-    }
-    const unsigned lane_off = (threadIdx.x & (kTabCopies - 1)) * 16u;
-    double2* exp_tab = reinterpret_cast<double2*>(smem_raw + kTabSmemBytes);
-    for (int e = threadIdx.x; e < kExpEntries; e += THREADS) {
-        double2 v;
-        if (e == 0) v = make_double2(__longlong_as_double(0xFFF0000000000000LL), 0.0);                       // zero / subnormal derivative
-        else if (e >= 2046) v = make_double2(__longlong_as_double(0x7FF8000000000000LL), 0.0);                // inf, NaN, or a set sign bit
-        else v = make_double2(__dmul_rn((double)(e + 1), LYAP_LN2HI), __fma_rn((double)(e + 1), LYAP_LN2LO, LYAP_KLO_BIAS));
-        exp_tab[e] = v;
-    }
-    __syncthreads();   // both tables are read across warps from the first logarithm on (at once when warmup == 0)
+// The orbits and stores of one warp-tile: the 32*P pixels from pixel `tile0` of the launch on.  KG == 0: patterns
+// dispatched at run time; KG > 0: WU_PATS / ACC_PATS are the group patterns of the warm-up and accumulation regions.
+template <int P, bool HAS_C, int UNROLL, int KG, unsigned long long WU_PATS, unsigned long long ACC_PATS>
+__device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long tile0, double* __restrict__ out64,
+                                           float* __restrict__ out32, double* stage, unsigned lane_off,
+                                           unsigned long long& my_steps) {
+    const int lane = threadIdx.x & 31;
+    const long long idx0 = tile0 + (long long)lane * P;
+    double x[P], lyap[P], rA[P], rB[P], lam[P];
+    const double rC = a.c_value;
+    int valid[P];
+    bool done[P], careful_only[P];
 
-    unsigned long long my_steps = 0;
-    // Work is dealt out per WARP: warp-tile t is the 32*P consecutive pixels from t*32*P, and the warps of the grid take
-    // them round-robin, warp index first (tile t goes to warp t / gridDim of block t % gridDim), so that when the tiles
-    // do not fill a whole number of rounds every SM gets the same mix of busier and idler warps.  (Dealt out per block,
-    // a frame of 9.1 rounds costs 10; this way it costs about 9.1.)
-    const long long tile_px = 32LL * P;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long warps_in_grid = (long long)gridDim.x * (THREADS / 32);
-    const int n_regions = 2;
-
-    for (long long tile = (long long)warp * gridDim.x + blockIdx.x; tile * tile_px < a.n_pixels; tile += warps_in_grid) {
-        const long long idx0 = tile * tile_px + (long long)lane * P;
-        double x[P], lyap[P], rA[P], rB[P], lam[P];
-        const double rC = a.c_value;
-        int valid[P];
-        bool done[P], careful_only[P];
-
-        {
-            long long row = idx0 / a.width;
-            int col = (int)(idx0 - row * a.width);
-            row += a.row_begin;
+    {
+        long long row = idx0 / a.width;
+        int col = (int)(idx0 - row * a.width);
+        row += a.row_begin;
 #pragma unroll
-            for (int p = 0; p < P; ++p) {
-                const bool inside = idx0 + p < a.n_pixels;
-                rB[p] = __dadd_rn(a.min_y, __dmul_rn(a.dy, (double)(int)row));   // :42
-                rA[p] = __dadd_rn(a.min_x, __dmul_rn(a.dx, (double)col));        // :45
-                x[p] = 0.5;                                                       // :31,52
-                lyap[p] = 0.0;
-                valid[p] = 0;
-                lam[p] = -5.0;
-                done[p] = !inside || rA[p] <= 0.0 || rB[p] <= 0.0;                // :47-50
-                careful_only[p] = !(ordinary_param(rA[p]) && ordinary_param(rB[p]) && a.fast_ok_c);
-                if (++col == a.width) {
-                    col = 0;
-                    ++row;
-                }
+        for (int p = 0; p < P; ++p) {
+            const bool inside = idx0 + p < a.n_pixels;
+            rB[p] = __dadd_rn(a.min_y, __dmul_rn(a.dy, (double)(int)row));   // :42
+            rA[p] = __dadd_rn(a.min_x, __dmul_rn(a.dx, (double)col));        // :45
+            x[p] = 0.5;                                                       // :31,52
+            lyap[p] = 0.0;
+            valid[p] = 0;
+            lam[p] = -5.0;
+            done[p] = !inside || rA[p] <= 0.0 || rB[p] <= 0.0;                // :47-50
+            careful_only[p] = !(ordinary_param(rA[p]) && ordinary_param(rB[p]) && a.fast_ok_c);
+            if (++col == a.width) {
+                col = 0;
+                ++row;
             }
         }
+    }
 
-        for (int region = 0; region < n_regions; ++region) {
-            const bool acc = region == 1;
-            const int nsteps = acc ? a.iterations : a.warmup;
-            const int word0 = acc ? a.acc_word0 : 0;
-            const int wrap = acc ? a.acc_wrap : a.wu_wrap;
-            if constexpr (KG > 0) {
-                // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
-                // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code)
-                constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = 2, CS = CB * BS * REP;
-                const unsigned* sel = a.sel + word0;
-                int s = 0;
-                while (s < nsteps) {
-                    bool all_done = true;
-#pragma unroll
-                    for (int p = 0; p < P; ++p) all_done = all_done && done[p];
-                    if (__all_sync(0xFFFFFFFFu, all_done)) break;
-                    const int left = nsteps - s;
-                    const int n = left >= CS ? CS : (left >= CB * BS ? CB * BS : (left >= BS ? left / BS * BS : left));
-                    double sx[P], sl[P];
-#pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        sx[p] = x[p];
-                        sl[p] = lyap[p];
-                    }
-                    if (left >= CS) {             // CB whole periods, straight-line, REP times
-#pragma unroll 1
-                        for (int rep = 0; rep < REP; ++rep) {
-#pragma unroll
-                            for (int b = 0; b < CB; ++b) {
-                                if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
-                                else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
-                            }
-                        }
-                    } else if (left >= CB * BS) { // one straight-line block
-#pragma unroll
-                        for (int b = 0; b < CB; ++b) {
-                            if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
-                            else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
-                        }
-                    } else if (left >= BS) {      // the last few whole periods
-#pragma unroll 1
-                        for (int b = 0; b < n / BS; ++b) {
-                            if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
-                            else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
-                        }
-                    } else {                      // less than one period: one step at a time
-#pragma unroll 1
-                        for (int j = s; j < nsteps; ++j) {
-                            const unsigned code = (sel[(j / kStepsPerWord) % wrap] >> (2 * (j & (kStepsPerWord - 1)))) & 3u;
-                            if (acc) fast_group<P, true, HAS_C, 1>(x, lyap, rA, rB, rC, code, lane_off);
-                            else fast_group<P, false, HAS_C, 1>(x, lyap, rA, rB, rC, code, lane_off);
-                        }
-                    }
-#pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        if (done[p]) continue;
-                        const bool regular = !careful_only[p] && in_unit_interval(x[p]) && isfinite(lyap[p]);
-                        if (regular) {
-                            if (acc) valid[p] += n;
-                            my_steps += (unsigned long long)n;
-                        } else {
-                            PixelState ps{sx[p], sl[p], valid[p]};
-                            const bool dead = acc ? careful_steps<true>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps)
-                                                  : careful_steps<false>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps);
-                            x[p] = ps.x;
-                            lyap[p] = ps.lyap;
-                            valid[p] = ps.valid;
-                            if (dead) {
-                                done[p] = true;
-                                lam[p] = ps.valid > 0 ? __ddiv_rn(ps.lyap, __dmul_rn((double)ps.valid, LYAP_LN2)) : -5.0;   // :84-85
-                                x[p] = 0.25;
-                            }
-                        }
-                    }
-                    s += n;
-                }
-                continue;
-            }
-            // generic walk: the selector words one after the other, exit tests after every second full word
+    for (int region = 0; region < 2; ++region) {
+        const bool acc = region == 1;
+        const int nsteps = acc ? a.iterations : a.warmup;
+        const int word0 = acc ? a.acc_word0 : 0;
+        const int wrap = acc ? a.acc_wrap : a.wu_wrap;
+        if constexpr (KG > 0) {
+            // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
+            // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code)
+            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = 2, CS = CB * BS * REP;
             const unsigned* sel = a.sel + word0;
-            int s = 0, wi = 0;
+            int s = 0;
             while (s < nsteps) {
                 bool all_done = true;
 #pragma unroll
                 for (int p = 0; p < P; ++p) all_done = all_done && done[p];
                 if (__all_sync(0xFFFFFFFFu, all_done)) break;
-
                 const int left = nsteps - s;
-                const int n = left >= 2 * kStepsPerWord ? 2 * kStepsPerWord : (left >= kStepsPerWord ? kStepsPerWord : left);
+                const int n = left >= CS ? CS : (left >= CB * BS ? CB * BS : (left >= BS ? left / BS * BS : left));
                 double sx[P], sl[P];
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     sx[p] = x[p];
                     sl[p] = lyap[p];
                 }
+                if (left >= CS) {             // CB whole periods, straight-line, REP times
 #pragma unroll 1
-                for (int k = 0; k < n; k += kStepsPerWord) {
-                    const unsigned word = sel[wi];
-                    if (++wi == wrap) wi = 0;
-                    const int m = min(kStepsPerWord, n - k);
-                    if (acc) fast_chunk<P, true, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
-                    else fast_chunk<P, false, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
+                    for (int rep = 0; rep < REP; ++rep) {
+#pragma unroll
+                        for (int b = 0; b < CB; ++b) {
+                            if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
+                            else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
+                        }
+                    }
+                } else if (left >= CB * BS) { // one straight-line block
+#pragma unroll
+                    for (int b = 0; b < CB; ++b) {
+                        if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
+                        else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
+                    }
+                } else if (left >= BS) {      // the last few whole periods
+#pragma unroll 1
+                    for (int b = 0; b < n / BS; ++b) {
+                        if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
+                        else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
+                    }
+                } else {                      // less than one period: one step at a time
+#pragma unroll 1
+                    for (int j = s; j < nsteps; ++j) {
+                        const unsigned code = (sel[(j / kStepsPerWord) % wrap] >> (2 * (j & (kStepsPerWord - 1)))) & 3u;
+                        if (acc) fast_group<P, true, HAS_C, 1>(x, lyap, rA, rB, rC, code, lane_off);
+                        else fast_group<P, false, HAS_C, 1>(x, lyap, rA, rB, rC, code, lane_off);
+                    }
                 }
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     if (done[p]) continue;
-                    // an irregular derivative (zero, subnormal, non-finite) has made the sum non-finite through the exponent table
                     const bool regular = !careful_only[p] && in_unit_interval(x[p]) && isfinite(lyap[p]);
                     if (regular) {
                         if (acc) valid[p] += n;
@@ -497,58 +419,157 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
                         if (dead) {
                             done[p] = true;
                             lam[p] = ps.valid > 0 ? __ddiv_rn(ps.lyap, __dmul_rn((double)ps.valid, LYAP_LN2)) : -5.0;   // :84-85
-                            x[p] = 0.25;   // keep the abandoned lane's arithmetic tame
+                            x[p] = 0.25;
                         }
                     }
                 }
                 s += n;
             }
+            continue;
         }
+        // generic walk: the selector words one after the other, exit tests after every second full word
+        const unsigned* sel = a.sel + word0;
+        int s = 0, wi = 0;
+        while (s < nsteps) {
+            bool all_done = true;
+#pragma unroll
+            for (int p = 0; p < P; ++p) all_done = all_done && done[p];
+            if (__all_sync(0xFFFFFFFFu, all_done)) break;
+
+            const int left = nsteps - s;
+            const int n = left >= 2 * kStepsPerWord ? 2 * kStepsPerWord : (left >= kStepsPerWord ? kStepsPerWord : left);
+            double sx[P], sl[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                sx[p] = x[p];
+                sl[p] = lyap[p];
+            }
+#pragma unroll 1
+            for (int k = 0; k < n; k += kStepsPerWord) {
+                const unsigned word = sel[wi];
+                if (++wi == wrap) wi = 0;
+                const int m = min(kStepsPerWord, n - k);
+                if (acc) fast_chunk<P, true, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
+                else fast_chunk<P, false, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
+            }
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                if (done[p]) continue;
+                // an irregular derivative (zero, subnormal, non-finite) has made the sum non-finite through the exponent table
+                const bool regular = !careful_only[p] && in_unit_interval(x[p]) && isfinite(lyap[p]);
+                if (regular) {
+                    if (acc) valid[p] += n;
+                    my_steps += (unsigned long long)n;
+                } else {
+                    PixelState ps{sx[p], sl[p], valid[p]};
+                    const bool dead = acc ? careful_steps<true>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps)
+                                          : careful_steps<false>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps);
+                    x[p] = ps.x;
+                    lyap[p] = ps.lyap;
+                    valid[p] = ps.valid;
+                    if (dead) {
+                        done[p] = true;
+                        lam[p] = ps.valid > 0 ? __ddiv_rn(ps.lyap, __dmul_rn((double)ps.valid, LYAP_LN2)) : -5.0;   // :84-85
+                        x[p] = 0.25;   // keep the abandoned lane's arithmetic tame
+                    }
+                }
+            }
+            s += n;
+        }
+    }
 
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            if (!done[p]) lam[p] = valid[p] > 0 ? __ddiv_rn(lyap[p], __dmul_rn((double)valid[p], LYAP_LN2)) : -5.0;
-        }
+    for (int p = 0; p < P; ++p) {
+        if (!done[p]) lam[p] = valid[p] > 0 ? __ddiv_rn(lyap[p], __dmul_rn((double)valid[p], LYAP_LN2)) : -5.0;
+    }
 
-        // stores: each warp's 32*P consecutive values go through the warp's own staging row in shared memory, so that every
-        // lane writes 16 bytes and a store instruction covers consecutive 512-byte runs whatever P is (no block-wide barrier:
-        // warps stay out of step with each other); a ragged last tile or a misaligned output pointer takes plain stores
-        const long long tile0 = tile * tile_px;
-        const bool full_tile = tile0 + tile_px <= a.n_pixels;
-        double* stage = reinterpret_cast<double*>(smem_raw + kExactSmemBytes) + warp * (32 * P);
-        if (out64) {
-            if (full_tile && ((reinterpret_cast<uintptr_t>(out64 + tile0) & 15) == 0)) {
-                __syncwarp();   // the row is free (this warp's reads of the previous tile are done)
+    // stores: each warp's 32*P consecutive values go through the warp's own staging row in shared memory, so that every
+    // lane writes 16 bytes and a store instruction covers consecutive 512-byte runs whatever P is (no block-wide barrier:
+    // warps stay out of step with each other); a ragged last tile or a misaligned output pointer takes plain stores
+    const bool full_tile = tile0 + 32 * P <= a.n_pixels;
+    if (out64) {
+        if (full_tile && ((reinterpret_cast<uintptr_t>(out64 + tile0) & 15) == 0)) {
+            __syncwarp();   // the row is free (this warp's reads of the previous tile are done)
 #pragma unroll
-                for (int p = 0; p < P; ++p) stage[lane * P + p] = lam[p];
-                __syncwarp();
-                double2* dst = reinterpret_cast<double2*>(out64 + tile0);
-                const double2* src = reinterpret_cast<const double2*>(stage);
+            for (int p = 0; p < P; ++p) stage[lane * P + p] = lam[p];
+            __syncwarp();
+            double2* dst = reinterpret_cast<double2*>(out64 + tile0);
+            const double2* src = reinterpret_cast<const double2*>(stage);
 #pragma unroll
-                for (int i = lane; i < 16 * P; i += 32) dst[i] = src[i];
-            } else {
+            for (int i = lane; i < 16 * P; i += 32) dst[i] = src[i];
+        } else {
 #pragma unroll
-                for (int p = 0; p < P; ++p)
-                    if (idx0 + p < a.n_pixels) out64[idx0 + p] = lam[p];
-            }
+            for (int p = 0; p < P; ++p)
+                if (idx0 + p < a.n_pixels) out64[idx0 + p] = lam[p];
         }
-        if (out32) {
-            if (full_tile && ((reinterpret_cast<uintptr_t>(out32 + tile0) & 15) == 0)) {
-                float* stage32 = reinterpret_cast<float*>(stage);
-                __syncwarp();
+    }
+    if (out32) {
+        if (full_tile && ((reinterpret_cast<uintptr_t>(out32 + tile0) & 15) == 0)) {
+            float* stage32 = reinterpret_cast<float*>(stage);
+            __syncwarp();
 #pragma unroll
-                for (int p = 0; p < P; ++p) stage32[lane * P + p] = (float)lam[p];
-                __syncwarp();
-                float4* dst = reinterpret_cast<float4*>(out32 + tile0);
-                const float4* src = reinterpret_cast<const float4*>(stage32);
+            for (int p = 0; p < P; ++p) stage32[lane * P + p] = (float)lam[p];
+            __syncwarp();
+            float4* dst = reinterpret_cast<float4*>(out32 + tile0);
+            const float4* src = reinterpret_cast<const float4*>(stage32);
 #pragma unroll
-                for (int i = lane; i < 8 * P; i += 32) dst[i] = src[i];
-            } else {
+            for (int i = lane; i < 8 * P; i += 32) dst[i] = src[i];
+        } else {
 #pragma unroll
-                for (int p = 0; p < P; ++p)
-                    if (idx0 + p < a.n_pixels) out32[idx0 + p] = (float)lam[p];
-            }
+            for (int p = 0; p < P; ++p)
+                if (idx0 + p < a.n_pixels) out32[idx0 + p] = (float)lam[p];
         }
+    }
+}
+
+// Body shared by the library's generic kernel (KG == 0) and by a specialised instance (KG > 0).
+template <int P, int THREADS, bool HAS_C, int UNROLL, int KG, unsigned long long WU_PATS, unsigned long long ACC_PATS>
+__device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* __restrict__ out64, float* __restrict__ out32,
+                  unsigned long long* __restrict__ steps_out) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    lyap_logtab_entry* tab_all = reinterpret_cast<lyap_logtab_entry*>(smem_raw);
+    // every entry is read once and written to its copies in an order that differs by lane, so that the 8 lanes of a
+    // quarter warp write to 8 bank groups
+    for (int e = threadIdx.x; e < LYAP_LOG_BINS; e += THREADS) {
+        lyap_logtab_entry t = g_lyap_logtab[e];
+        t.invc = __hiloint2double(__double2hiint(t.invc) + 0x3FF00000, __double2loint(t.invc));   // see log_fast
+#pragma unroll
+        for (int c = 0; c < kTabCopies; ++c) tab_all[e * kTabCopies + ((threadIdx.x + c) & (kTabCopies - 1))] = t;
+    }
+    const unsigned lane_off = (threadIdx.x & (kTabCopies - 1)) * 16u;
+    double2* exp_tab = reinterpret_cast<double2*>(smem_raw + kTabSmemBytes);
+    for (int e = threadIdx.x; e < kExpEntries; e += THREADS) {
+        double2 v;
+        if (e == 0) v = make_double2(__longlong_as_double(0xFFF0000000000000LL), 0.0);                       // zero / subnormal derivative
+        else if (e >= 2046) v = make_double2(__longlong_as_double(0x7FF8000000000000LL), 0.0);                // inf, NaN, or a set sign bit
+        else v = make_double2(__dmul_rn((double)(e + 1), LYAP_LN2HI), __fma_rn((double)(e + 1), LYAP_LN2LO, LYAP_KLO_BIAS));
+        exp_tab[e] = v;
+    }
+    unsigned long long my_steps = 0;
+    // Work is dealt out to blocks round-robin (tile t to block t % gridDim), first a.wide_tiles warp-tiles of 32*P pixels,
+    // then the rest of the frame in tiles of 32 pixels; a block's tiles go round its four schedulers (a warp's scheduler is
+    // warp % 4), and a warp that is done takes its scheduler's next tile from a counter in shared memory.  Warps whose orbits
+    // leave (0,1) early so take more tiles, and the small ones at the end fill what the wide ones leave ragged: a scheduler's
+    // time is its pixels times a constant whatever its warps' shapes (2200 steps: 147 / 245 / 350 / 456 us for 1 / 2 / 3 / 4
+    // warps of 3 pixels a thread, 58 / 93 / 123 / 158 us for 1 / 2 / 3 / 4 of one).  With one counter a block the first
+    // scheduler to be done takes all small tiles of a frame of one round: 512 x 512 in 0.301 instead of 0.287 ms.
+    __shared__ unsigned next_unit[4];   // the first units are taken as unit == warp
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x < 4) next_unit[threadIdx.x] = THREADS / 32 + threadIdx.x;
+    __syncthreads();   // the counters, and both tables, which are read across warps from the first logarithm on
+    const long long wide_of_block = a.wide_tiles > blockIdx.x ? (a.wide_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
+    double* stage = reinterpret_cast<double*>(smem_raw + kExactSmemBytes) + warp * (32 * P);
+    for (unsigned unit = warp;;) {
+        if (unit < wide_of_block) {
+            const long long tile = (long long)unit * gridDim.x + blockIdx.x;
+            exact_tile<P, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, tile * (32LL * P), out64, out32, stage, lane_off, my_steps);
+        } else {
+            const long long at = a.wide_tiles * (32LL * P) + ((unit - wide_of_block) * gridDim.x + blockIdx.x) * 32;
+            if (at >= a.n_pixels) break;
+            exact_tile<1, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, at, out64, out32, stage, lane_off, my_steps);
+        }
+        if (lane == 0) unit = atomicAdd(&next_unit[warp & 3], 4u);
+        unit = __shfl_sync(0xFFFFFFFFu, unit, 0);
     }
 
     if (steps_out) {

@@ -251,7 +251,7 @@ int sequence_group_period(const LambdaArgs& a, unsigned long long* wu_pats, unsi
 // Launches the specialised instance when there is one (or when compiling one now is worth it).
 // mode: 0 never, 1 when the work seen for this sequence passes a threshold, 2 always.
 // *launched tells whether a kernel was enqueued; false means "use the precompiled kernel".
-cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, int sm_count,
+cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, unsigned grid,
                                cudaStream_t st, int kind, int pixels_per_thread, int threads, size_t smem_bytes, int mode,
                                bool* launched) {
     *launched = false;
@@ -260,10 +260,6 @@ cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32,
     unsigned long long wu = 0, acc = 0;
     const int kg = sequence_group_period(a, &wu, &acc);
     if (kg == 0) return cudaSuccess;
-    const long long tile_px = (long long)threads * pixels_per_thread;
-    const long long tiles = (a.n_pixels + tile_px - 1) / tile_px;
-    const long long cap = kind == 0 ? sm_count : 4LL * sm_count;   // the exact kernel's shared tables allow one CTA per SM
-    const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
     char name[160];
     static const char* const kinds[4] = {"k_lambda_exact", "k_lambda_fast<FusedF64>", "k_lambda_fast<FusedF32>", "k_lambda_fast<OrbitF64>"};
 
@@ -290,7 +286,7 @@ cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32,
                 fn = e.fn;
             }
             if (!fn) break;   // could not be loaded (lyap_jit_note says why): run-time compilation or the generic kernel
-            if (tiles > 0) {
+            if (grid > 0) {
                 const CUresult r = driver().launch_kernel(fn, grid, 1, 1, (unsigned)threads, 1, 1, (unsigned)smem_bytes, (CUstream)st, params, nullptr);
                 if (r != CUDA_SUCCESS) {
                     std::lock_guard<std::mutex> lk(g_mu);
@@ -350,7 +346,7 @@ cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32,
         fn = e.fn;
     }
     if (!fn) return cudaSuccess;
-    if (tiles <= 0) { *launched = true; return cudaSuccess; }
+    if (grid == 0) { *launched = true; return cudaSuccess; }
     const CUresult r = driver().launch_kernel(fn, grid, 1, 1, (unsigned)threads, 1, 1, (unsigned)smem_bytes, (CUstream)st, params, nullptr);
     if (r != CUDA_SUCCESS) {
         std::lock_guard<std::mutex> lk(g_mu);

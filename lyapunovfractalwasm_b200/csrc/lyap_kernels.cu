@@ -19,48 +19,19 @@
 
 namespace lyap {
 
-template <int P, int THREADS, bool HAS_C, int UNROLL>
-static cudaError_t launch_exact_variant(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                        int sm_count, cudaStream_t st) {
-    auto kern = k_lambda_exact<P, THREADS, HAS_C, UNROLL>;
-    constexpr size_t smem = exact_smem_bytes(THREADS, P);
+constexpr int kExactThreads = 512, kExactPixels = 3;   // measured best shape of the wide tiles on large frames
+
+template <bool HAS_C>
+static cudaError_t launch_exact_generic(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
+                                        unsigned grid, cudaStream_t st) {
+    auto kern = k_lambda_exact<kExactPixels, kExactThreads, HAS_C, 2>;
+    constexpr size_t smem = exact_smem_bytes(kExactThreads, kExactPixels);
     // the attribute is per device and cheap to set; doing it on every launch keeps this thread- and device-safe
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const long long tile_px = (long long)THREADS * P;     // one round of a block's warps (work is dealt out per warp)
-    const long long tiles = (a.n_pixels + tile_px - 1) / tile_px;
-    if (tiles <= 0) return cudaSuccess;
-    const int grid = (int)(tiles < sm_count ? tiles : sm_count);
-    kern<<<grid, THREADS, smem, st>>>(a, out64, out32, steps);
-    static const char* const names[2] = {"k_lambda_exact<2,512> (generic: patterns dispatched every 2 steps)",
-                                         "k_lambda_exact<3,512> (generic: patterns dispatched every 2 steps)"};
-    note_lambda_kernel(names[P - 2]);
+    kern<<<grid, kExactThreads, smem, st>>>(a, out64, out32, steps);
+    note_lambda_kernel("k_lambda_exact<3,512> (generic: patterns dispatched every 2 steps)");
     return cudaGetLastError();
-}
-
-// Pixels per thread for a launch of n pixels.  Large frames: 3 (measured best on B200).  A frame of only a few rounds of
-// warp-tiles is dominated by its last, partly filled round, in which the few warps still working run faster than in a
-// full round but not in proportion (one warp alone reaches under half of its scheduler's fp64 rate); the shape with the
-// smaller estimate of (full rounds + last round) x per-pixel cost is taken.  `spec`: the shapes run as instances made for
-// the sequence, which are faster.
-static int exact_pixels_per_thread(long long n_pixels, int sm_count, bool spec) {
-    const int cand[2] = {3, 2};
-    const double cost[2] = {spec ? 0.92 : 1.0, spec ? 0.95 : 1.035};
-    const double warps = (double)sm_count * 16.0;
-    int best = 3;
-    double best_t = 1e300;
-    for (int i = 0; i < 2; ++i) {
-        const double tiles = (double)((n_pixels + 32LL * cand[i] - 1) / (32LL * cand[i]));
-        const double rounds = tiles / warps;
-        const double full = (double)(long long)rounds, frac = rounds - full;
-        const double last = frac <= 0.0 ? 0.0 : (frac < 0.45 ? 0.45 : frac);
-        const double t = (full + last) * cand[i] * cost[i];
-        if (t < best_t * 0.999) {
-            best_t = t;
-            best = cand[i];
-        }
-    }
-    return best;
 }
 
 // LYAP_JIT: 0 never compile at run time, 1 (default) once enough work with a sequence has been seen, 2 at once.
@@ -73,29 +44,26 @@ static int spec_mode() {
     return (jit < 0 ? 0 : (jit > 2 ? 2 : jit)) | (pre ? kSpecUsePrebuilt : 0);
 }
 
-cudaError_t launch_lambda_exact(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
+cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* out32, unsigned long long* steps,
                                 int sm_count, cudaStream_t st) {
+    if (args.n_pixels <= 0) return cudaSuccess;
+    LambdaArgs a = args;
     bool has_c = false;
     const int words = a.acc_word0 + (a.iterations > 0 ? min(a.acc_wrap, (a.iterations - 1) / kStepsPerWord + 1) : 0);
     for (int i = 0; i < words; ++i) has_c = has_c || (a.sel[i] & 0xAAAAAAAAu);
-#define LYAP_VARIANT(P, T, U)                                                                    \
-    (has_c ? launch_exact_variant<P, T, true, U>(a, out64, out32, steps, sm_count, st)            \
-           : launch_exact_variant<P, T, false, U>(a, out64, out32, steps, sm_count, st))
+    // wide tiles in whole rounds over the device's schedulers (4 an SM); 2 to 5 tiles of 32 pixels a scheduler are left to
+    // even out the end
+    const long long wide_px = 32LL * kExactPixels, schedulers = 4LL * sm_count;
+    a.wide_tiles = a.n_pixels > 64 * schedulers ? (a.n_pixels - 64 * schedulers) / (wide_px * schedulers) * schedulers : 0;
+    const long long warp_tiles = a.wide_tiles + (a.n_pixels - a.wide_tiles * wide_px + 31) / 32;
+    const unsigned grid = (unsigned)(warp_tiles < sm_count ? warp_tiles : sm_count);   // the shared tables allow one CTA per SM
     // a periodic sequence can run an instance of this kernel made for its patterns
-    const int mode = spec_mode();
-    unsigned long long wu_pats = 0, acc_pats = 0;
-    const bool spec = mode != 0 && sequence_group_period(a, &wu_pats, &acc_pats) > 0;
-    const int ppt = exact_pixels_per_thread(a.n_pixels, sm_count, spec);
-    {
-        bool launched = false;
-        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, sm_count, st, 0, ppt, 512, exact_smem_bytes(512, ppt),
-                                                 mode, &launched);
-        if (e != cudaSuccess) return e;
-        if (launched) return cudaSuccess;
-    }
-    if (ppt == 2) return LYAP_VARIANT(2, 512, 2);
-    return LYAP_VARIANT(3, 512, 2);
-#undef LYAP_VARIANT
+    bool launched = false;
+    const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads,
+                                             exact_smem_bytes(kExactThreads, kExactPixels), spec_mode(), &launched);
+    if (e != cudaSuccess || launched) return e;
+    return has_c ? launch_exact_generic<true>(a, out64, out32, steps, grid, st)
+                 : launch_exact_generic<false>(a, out64, out32, steps, grid, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -633,7 +601,9 @@ static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, floa
                                         int sm_count, cudaStream_t st, int kind, int spec_ppt, const char* generic_name) {
     {   // a periodic sequence can run an instance made for its patterns (same switches as the exact kernel)
         bool launched = false;
-        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, sm_count, st, kind, spec_ppt, 512, 0, spec_mode(), &launched);
+        const long long px = 512LL * spec_ppt, spec_tiles = (a.n_pixels + px - 1) / px;
+        const unsigned spec_grid = (unsigned)(spec_tiles < 4LL * sm_count ? spec_tiles : 4LL * sm_count);
+        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, spec_grid, st, kind, spec_ppt, 512, 0, spec_mode(), &launched);
         if (e != cudaSuccess) return e;
         if (launched) return cudaSuccess;
     }
