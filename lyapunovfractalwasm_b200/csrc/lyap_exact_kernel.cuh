@@ -140,13 +140,43 @@ __device__ __forceinline__ double log_fast(double d, unsigned lane_off) {
     return __dadd_rn(hi, s);
 }
 
-// careful_chunk for steps [first, first + n) of a region whose selector words start at `sel`.
+// careful_chunk for steps [first, first + n) of a region whose selector words start at `sel` (n <= 64).
+// An orbit that has fallen below 2^-600 and whose parameters (positive: the others are sentinels) are at most 256 stays
+// below 2^-88 for these steps, where 1 - 2x and 1 - x round to 1: the derivative is the parameter itself, with one of at
+// most three logarithms, and a step is a multiplication, an addition and the exit test.  That is how nearly every orbit of
+// a frame over [0,4]^2 that ends does end (x runs down to zero where rA*rB < 1), a whole region's after one another.
+// Measured, 800 x 800 over [0.01,3.99]^2, "AB" 100 + 1000: 0.745 -> 0.702 ms (0.645 for a window without exits).
 template <bool ACC>
 __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB, double rC, const unsigned* sel, int wrap, int first,
                                            int n, unsigned long long* steps) {
     bool dead = false;
     int j = first;
     const int end = first + n;
+    if (ps->x < 0x1p-600 && rA <= 256.0 && rB <= 256.0) {
+        const unsigned codes = rC > 0.0 && rC <= 256.0 ? 3 : 2;   // parameters that may be used this way
+        double x = ps->x, lyap = ps->lyap, zA = 0.0, zB = 0.0, zC = 0.0;
+        if (ACC) {
+            zA = lyap_log_tab(rA, g_lyap_logtab, 1);
+            zB = lyap_log_tab(rB, g_lyap_logtab, 1);
+            zC = lyap_log_tab(rC, g_lyap_logtab, 1);
+        }
+        while (j < end && !dead) {   // leaves at a step that uses another one: the rest is walked below
+            const int in_word = j & (kStepsPerWord - 1);
+            const int stop = min(j + kStepsPerWord - in_word, end);
+            for (unsigned word = sel[(j / kStepsPerWord) % wrap] >> (2 * in_word); j < stop && !dead; ++j, word >>= 2) {
+                const unsigned code = word & 3u;
+                if (code >= codes) break;
+                x = __dmul_rn(code == 0 ? rA : (code == 1 ? rB : rC), x);
+                if (ACC) lyap = __dadd_rn(lyap, code == 0 ? zA : (code == 1 ? zB : zC));
+                dead = !(x > 0.0);
+            }
+            if (j < stop) break;
+        }
+        if (ACC) ps->valid += j - first;
+        *steps += (unsigned long long)(j - first);
+        ps->x = x;
+        ps->lyap = lyap;
+    }
     while (j < end && !dead) {
         const int in_word = j & (kStepsPerWord - 1);
         const int m = min(kStepsPerWord - in_word, end - j);

@@ -165,6 +165,22 @@ def test_every_tile_of_a_launch_is_walked_once(engine, port, kernel_path, path, 
         assert np.array_equal(r["lambda32"].view(np.uint32), lam.astype(np.float32).view(np.uint32))
 
 
+@pytest.mark.parametrize("kw", [
+    dict(sequence="AB", max_x=1.1, max_y=1.1), dict(sequence="BBBBBBAAAAAA", max_x=4.0, max_y=0.3),
+    dict(sequence="ABB" * 15 + "A", max_x=300.0, max_y=0.01),                           # some parameters above the rule's 256
+    dict(sequence="ABC", max_x=1.0, max_y=1.0, c=0.3), dict(sequence="AABBC", max_x=0.5, max_y=0.5, c=300.0),
+    dict(sequence="ABABABABABABABC", max_x=0.5, max_y=0.5, c=-1.0), dict(sequence="AB", max_x=0.5, max_y=0.5, c=-1.0),
+], ids=lambda kw: "%s_%s" % (kw["sequence"][:6], kw.get("c")))
+@pytest.mark.parametrize("path", ["jit", "generic"])
+def test_orbits_that_run_down_to_zero(engine, port, kernel_path, path, kw):
+    """Exits by underflow, in warm-up and in accumulation, at every place of a chunk: bits and executed steps."""
+    kernel_path(path)
+    kw = dict(dict(min_x=0.003, min_y=0.002, width=97, height=41, iterations=1300, warmup=150), **kw)
+    r = engine.render(L.make_params(**kw), want=("lambda",))
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps
+
+
 def test_step_count_edges(engine, port):
     for warmup, iterations in ((0, 1), (0, 16), (1, 0), (16, 16), (17, 31), (15, 33), (0, 0)):
         kw = dict(min_x=2.6, max_x=4.0, min_y=2.7, max_y=3.9, width=40, height=12, sequence="BA", iterations=iterations,
