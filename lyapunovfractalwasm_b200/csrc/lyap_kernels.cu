@@ -598,12 +598,15 @@ namespace lyap {
 
 template <typename FL, int P>
 static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                        int sm_count, cudaStream_t st, int kind, int spec_ppt, const char* generic_name) {
+                                        int sm_count, cudaStream_t st, int kind, int spec_ppt, int spec_threads,
+                                        const char* generic_name) {
     {   // a periodic sequence can run an instance made for its patterns (same switches as the exact kernel)
         bool launched = false;
-        const long long px = 512LL * spec_ppt, spec_tiles = (a.n_pixels + px - 1) / px;
-        const unsigned spec_grid = (unsigned)(spec_tiles < 4LL * sm_count ? spec_tiles : 4LL * sm_count);
-        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, spec_grid, st, kind, spec_ppt, 512, 0, spec_mode(), &launched);
+        const long long px = (long long)spec_threads * spec_ppt, spec_tiles = (a.n_pixels + px - 1) / px;
+        const long long cap = 2048 / spec_threads * sm_count;
+        const unsigned spec_grid = (unsigned)(spec_tiles < cap ? spec_tiles : cap);
+        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, spec_grid, st, kind, spec_ppt, spec_threads, 0, spec_mode(),
+                                                 &launched);
         if (e != cudaSuccess) return e;
         if (launched) return cudaSuccess;
     }
@@ -622,20 +625,22 @@ static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, floa
     return cudaGetLastError();
 }
 
-// measured best shapes for the instances made for a sequence: fused fp64 4 pixels/thread, fp32 2, same-orbit fp64 3; 512 threads
+// measured best shapes for the instances made for a sequence: fused fp64 4 pixels/thread, same-orbit fp64 3, of 512 threads;
+// fp32 2 of 256: 4096 x 2048 pixels of "AABAB" 200 + 2000 take 2.54 / 2.58 ms with 512 / 256 threads, but 2048 x 2048 over
+// [0.01,3.99]^2, where a block waits for its slowest orbits, 2.34 / 2.04
 cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                  int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<FusedF64, 4>(a, out64, out32, steps, sm_count, st, 1, 4, "k_lambda_fast<FusedF64,4,256> (generic)");
+    return launch_lambda_fast_t<FusedF64, 4>(a, out64, out32, steps, sm_count, st, 1, 4, 512, "k_lambda_fast<FusedF64,4,256> (generic)");
 }
 
 cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                  int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<FusedF32, 4>(a, out64, out32, steps, sm_count, st, 2, 2, "k_lambda_fast<FusedF32,4,256> (generic)");
+    return launch_lambda_fast_t<FusedF32, 4>(a, out64, out32, steps, sm_count, st, 2, 2, 256, "k_lambda_fast<FusedF32,4,256> (generic)");
 }
 
 cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                   int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<OrbitF64, 4>(a, out64, out32, steps, sm_count, st, 3, 3, "k_lambda_fast<OrbitF64,4,256> (generic)");
+    return launch_lambda_fast_t<OrbitF64, 4>(a, out64, out32, steps, sm_count, st, 3, 3, 512, "k_lambda_fast<OrbitF64,4,256> (generic)");
 }
 
 }  // namespace lyap
