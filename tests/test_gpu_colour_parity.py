@@ -106,3 +106,35 @@ def test_config4_colour_stage_on_a_band_with_given_minmax(engine, port):
     assert np.array_equal(d_rgba.to_host(np.uint8).reshape(rows - 2, W, 4), port.colorize(want_norm, 0)[1:-1])
     for b in (d_lam, d_norm, d_rgba, d_mm):
         b.free()
+
+
+# no more than 100: an angle's quadrant is a conversion to int, which CPU and GPU define differently from 2^31 on (the
+# angle is at most 6 pi t; infinities and 1e300 gave other bytes than the CPU's before and after)
+SPECIAL = [0.0, -0.0, 1.0, 0.5, 1e-310, 2.0 ** -301, 2.0 ** -300, 1.0 + 2.0 ** -52, 3.0, -0.25, 100.0, np.nan]
+
+
+@pytest.mark.parametrize("shape", [(1, 5), (2, 4), (3, 6), (9, 7), (255, 9), (256, 4), (257, 5), (258, 12), (513, 6)])
+def test_colour_kernel_edges_and_special_values(engine, port, shape):
+    """Every palette at widths around a block's 256 columns and heights around a strip's 4 rows; half of the frames carry
+    values a picture has none of, which take the general palette code: bytes equal the oracle's."""
+    w, h = shape
+    rng = np.random.default_rng(w * 100 + h)
+    for special in (False, True):
+        norm = rng.uniform(0.0, 1.0, size=(h, w))
+        if special:
+            at = rng.integers(0, h * w, size=max(1, h * w // 40))
+            norm.flat[at] = rng.choice(SPECIAL, size=at.size)
+        for palette in range(7):
+            assert np.array_equal(engine.colorize(norm, palette), port.colorize(norm, palette)), (special, palette)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 511, 512, 513, 303105])
+def test_normalise_edges_and_special_values(engine, port, n):
+    """Lengths around a block's round of pairs, values that are sentinels, special or the frame's own extremes."""
+    rng = np.random.default_rng(n)
+    for special in (False, True):
+        values = rng.uniform(-3.0, 1.2, size=n)
+        if special:
+            at = rng.integers(0, n, size=max(1, n // 5))
+            values[at] = rng.choice([-5.0, -4.0, -3.9999999, np.nan, np.inf, -np.inf, 0.0, 1e-310, -3.0, 1.2], size=at.size)
+        assert same_bits(engine.normalize_data(values), port.normalize(values)), special
