@@ -435,7 +435,7 @@ int lyap_glow_device(lyap_ctx* c, uint8_t* d_rgba, int32_t width, int32_t height
     if (int r = check_ctx(c)) return r;
     if (width < 1 || height < 1) return fail(LYAP_ERR_INVALID, "bad dimensions");
     if (!d_rgba || !d_scratch) return fail(LYAP_ERR_INVALID, "null pointer");
-    cudaError_t e = lyap::launch_glow(d_rgba, width, height, static_cast<double*>(d_scratch), c->sm_count, c->stream);
+    cudaError_t e = lyap::launch_glow(d_rgba, width, height, static_cast<double*>(d_scratch), c->stream);
     if (e != cudaSuccess) return fail_cuda(e, "glow launch");
     return LYAP_OK;
 }
@@ -611,7 +611,7 @@ int lyap_glow(lyap_ctx* c, const uint8_t* rgba_in, int32_t width, int32_t height
     if (int r = ensure(c, c->norm, n * 24)) return r;   // the blur's scratch shares the normalised-frame buffer
     cudaStream_t st = c->stream;
     CU(cudaMemcpyAsync(c->rgba.p, rgba_in, n * 4, cudaMemcpyHostToDevice, st));
-    cudaError_t e = lyap::launch_glow(static_cast<uint8_t*>(c->rgba.p), width, height, static_cast<double*>(c->norm.p), c->sm_count, st);
+    cudaError_t e = lyap::launch_glow(static_cast<uint8_t*>(c->rgba.p), width, height, static_cast<double*>(c->norm.p), st);
     if (e != cudaSuccess) return fail_cuda(e, "glow launch");
     CU(cudaMemcpyAsync(rgba_out, c->rgba.p, n * 4, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));

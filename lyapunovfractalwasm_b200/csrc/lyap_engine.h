@@ -58,7 +58,7 @@ cudaError_t launch_colorize(const double* norm, int width, long long rows, int r
                             int palette, unsigned char* rgba, int sm_count, cudaStream_t st);
 
 // glow on an RGBA8 canvas in place; scratch holds width*height*3 doubles
-cudaError_t launch_glow(unsigned char* canvas, int width, int height, double* scratch, int sm_count, cudaStream_t st);
+cudaError_t launch_glow(unsigned char* canvas, int width, int height, double* scratch, cudaStream_t st);
 
 // issue-rate micro-benchmarks; return thread-level instructions executed per launch
 cudaError_t launch_fp64_peak(double* sink, int sm_count, int iters, unsigned long long* instr, cudaStream_t st);

@@ -215,6 +215,14 @@ def test_glow_matches_the_cpu_restatement(engine, port):
     assert np.array_equal(engine.glow(tiny), port.glow(tiny))
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (1, 40), (40, 1), (287, 7), (288, 8), (289, 9), (35, 17), (128, 36), (129, 37), (613, 19)])
+def test_glow_at_the_edges_of_its_tiles(engine, port, shape):
+    """Widths around a block's 288 and 128 columns, heights around a strip's 8 rows, pictures smaller than the blur."""
+    w, h = shape
+    rgba = np.random.default_rng(w * 1000 + h).integers(0, 256, size=(h, w, 4), dtype=np.uint8)
+    assert np.array_equal(engine.glow(rgba), port.glow(rgba))
+
+
 def test_render_frames_batch_equals_frame_by_frame(engine, port):
     """lyap_render_frames (two buffer sets, copies on their own stream) against lyap_render frame by frame and the
     oracle: frames of different sizes and sequences, more frames than buffer sets, the same device listed twice."""
