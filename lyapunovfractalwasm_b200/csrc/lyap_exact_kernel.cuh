@@ -42,11 +42,6 @@ constexpr size_t kTabSmemBytes = (size_t)LYAP_LOG_BINS * kTabCopies * sizeof(lya
 constexpr int kExpEntries = 4096;
 constexpr size_t kExpSmemBytes = (size_t)kExpEntries * sizeof(double2);                              // 64 KB
 constexpr size_t kExactSmemBytes = kTabSmemBytes + kExpSmemBytes;
-// after the tables: one staging row per warp (32 * P doubles each) for 16-byte-per-lane stores of the results
-__host__ __device__ constexpr size_t exact_smem_bytes(int threads, int pixels_per_thread) {
-    return kExactSmemBytes + (size_t)threads * pixels_per_thread * sizeof(double);
-}
-
 __device__ __forceinline__ bool in_unit_interval(double x) { return x > 0.0 && x < 1.0; }
 
 // parameter values the chunked fast path may be used with: positive, finite, 2^-500 < r < 2^500
@@ -192,8 +187,7 @@ __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB,
 // so the scheduler has U*P log chains to interleave.  The sum is still accumulated in step order.
 // The warp-uniform parameter choice is a select (no branch, so the block stays one scheduling region).
 template <int P, bool ACC, bool HAS_C, int U>
-__device__ __forceinline__ void fast_group(double (&x)[P], double (&lyap)[P], const double (&rA)[P],
-                                           const double (&rB)[P], double rC, unsigned word, unsigned lane_off) {
+__device__ __forceinline__ void fast_group(double (&x)[P], double (&lyap)[P], double rA, const double (&rB)[P], double rC, unsigned word, unsigned lane_off) {
     double d[U][P];
 #pragma unroll
     for (int j = 0; j < U; ++j) {
@@ -201,7 +195,7 @@ __device__ __forceinline__ void fast_group(double (&x)[P], double (&lyap)[P], co
         const bool is_c = (word >> (2 * j + 1)) & 1u;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            double r = not_a ? rB[p] : rA[p];
+            double r = not_a ? rB[p] : rA;
             if (HAS_C) r = is_c ? rC : r;
             if (ACC) {
                 d[j][p] = half_derivative(r, x[p]);
@@ -226,15 +220,14 @@ __device__ __forceinline__ void fast_group(double (&x)[P], double (&lyap)[P], co
 // U steps whose parameter choices are known at compile time (PAT: 2 bits per step, 0 = A, 1 = B, 2 = C):
 // no selects, no per-step branches; every operand is fixed.
 template <int P, bool ACC, int U, unsigned PAT>
-__device__ __forceinline__ void fixed_group(double (&x)[P], double (&lyap)[P], const double (&rA)[P],
-                                            const double (&rB)[P], double rC, unsigned lane_off) {
+__device__ __forceinline__ void fixed_group(double (&x)[P], double (&lyap)[P], double rA, const double (&rB)[P], double rC, unsigned lane_off) {
     double d[U][P];
 #pragma unroll
     for (int j = 0; j < U; ++j) {
         const unsigned code = (PAT >> (2 * j)) & 3u;
 #pragma unroll
         for (int p = 0; p < P; ++p) {
-            const double r = code == 0 ? rA[p] : (code == 1 ? rB[p] : rC);
+            const double r = code == 0 ? rA : (code == 1 ? rB[p] : rC);
             if (ACC) {
                 d[j][p] = half_derivative(r, x[p]);
             }
@@ -265,7 +258,7 @@ __host__ __device__ constexpr unsigned spread_bits(unsigned m) {
 //   !HAS_C: idx has one bit per step (0 = A, 1 = B), U is 2 or 4.   HAS_C: idx is the raw 2-bit codes, U is 2.
 template <int P, bool ACC, bool HAS_C, int U>
 __device__ __forceinline__ void dispatch_group(double (&x)[P], double (&lyap)[P],
-                                               const double (&rA)[P], const double (&rB)[P], double rC, unsigned idx,
+                                               double rA, const double (&rB)[P], double rC, unsigned idx,
                                                unsigned lane_off) {
 #define LYAP_CASE_AB(N) \
     case N: fixed_group<P, ACC, U, spread_bits(N)>(x, lyap, rA, rB, rC, lane_off); break;
@@ -310,8 +303,7 @@ __device__ __forceinline__ unsigned compress_even_bits(unsigned w) {
 
 // n steps of selector word `word` (2 bits per step: 0 = A, 1 = B, 2 = C).
 template <int P, bool ACC, bool HAS_C, int UNROLL>
-__device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], const double (&rA)[P],
-                                           const double (&rB)[P], double rC, unsigned word, int n, unsigned lane_off) {
+__device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], double rA, const double (&rB)[P], double rC, unsigned word, int n, unsigned lane_off) {
     if (n == kStepsPerWord) {
         constexpr int U = HAS_C ? 2 : UNROLL;
         unsigned pat = HAS_C ? word : compress_even_bits(word);
@@ -332,7 +324,7 @@ __device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], co
 // With the KG patterns known at compile time (PATS: 4 bits per group = two 2-bit codes) a whole period is one
 // straight-line block: no dispatch at all.
 template <int P, bool ACC, int KG, unsigned long long PATS, int G = 0>
-__device__ __forceinline__ void period_block(double (&x)[P], double (&lyap)[P], const double (&rA)[P], const double (&rB)[P],
+__device__ __forceinline__ void period_block(double (&x)[P], double (&lyap)[P], double rA, const double (&rB)[P],
                                              double rC, unsigned lane_off) {
     if constexpr (G < KG) {
         fixed_group<P, ACC, 2, (unsigned)((PATS >> (4 * G)) & 15ull)>(x, lyap, rA, rB, rC, lane_off);
@@ -344,39 +336,28 @@ __host__ __device__ constexpr bool pats_use_c(unsigned long long pats) {
     return (pats & 0xAAAAAAAAAAAAAAAAull) != 0;
 }
 
-// The orbits and stores of one warp-tile: the 32*P pixels from pixel `tile0` of the launch on.  KG == 0: patterns
-// dispatched at run time; KG > 0: WU_PATS / ACC_PATS are the group patterns of the warm-up and accumulation regions.
+// The orbits and stores of one warp-tile: this lane's pixels (row + p, col), p < P, of the launch; a lane that is not
+// `inside` has none.  The pixels of a thread lie below one another: they share the column's parameter, one register pair
+// instead of P, which the instructions of an A step read one after the other; orbits that end do so at much the same time
+// in 32 columns, less so in 32 * P; and each store of a warp covers 32 neighbours.
+// KG == 0: patterns dispatched at run time; KG > 0: WU_PATS / ACC_PATS are the regions' group patterns.
 template <int P, bool HAS_C, int UNROLL, int KG, unsigned long long WU_PATS, unsigned long long ACC_PATS>
-__device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long tile0, double* __restrict__ out64,
-                                           float* __restrict__ out32, double* stage, unsigned lane_off,
-                                           unsigned long long& my_steps) {
-    const int lane = threadIdx.x & 31;
-    const long long idx0 = tile0 + (long long)lane * P;
-    double x[P], lyap[P], rA[P], rB[P], lam[P];
+__device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, int col, bool inside, double* __restrict__ out64,
+                                           float* __restrict__ out32, unsigned lane_off, unsigned long long& my_steps) {
+    double x[P], lyap[P], rB[P], lam[P];
+    const double rA = __dadd_rn(a.min_x, __dmul_rn(a.dx, (double)col));                          // :45
     const double rC = a.c_value;
     int valid[P];
     bool done[P], careful_only[P];
-
-    {
-        long long row = idx0 / a.width;
-        int col = (int)(idx0 - row * a.width);
-        row += a.row_begin;
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const bool inside = idx0 + p < a.n_pixels;
-            rB[p] = __dadd_rn(a.min_y, __dmul_rn(a.dy, (double)(int)row));   // :42
-            rA[p] = __dadd_rn(a.min_x, __dmul_rn(a.dx, (double)col));        // :45
-            x[p] = 0.5;                                                       // :31,52
-            lyap[p] = 0.0;
-            valid[p] = 0;
-            lam[p] = -5.0;
-            done[p] = !inside || rA[p] <= 0.0 || rB[p] <= 0.0;                // :47-50
-            careful_only[p] = !(ordinary_param(rA[p]) && ordinary_param(rB[p]) && a.fast_ok_c);
-            if (++col == a.width) {
-                col = 0;
-                ++row;
-            }
-        }
+    for (int p = 0; p < P; ++p) {
+        rB[p] = __dadd_rn(a.min_y, __dmul_rn(a.dy, (double)(int)(a.row_begin + row + p)));       // :42
+        x[p] = 0.5;                                                                               // :31,52
+        lyap[p] = 0.0;
+        valid[p] = 0;
+        lam[p] = -5.0;
+        done[p] = !inside || rA <= 0.0 || rB[p] <= 0.0;                                           // :47-50
+        careful_only[p] = !(ordinary_param(rA) && ordinary_param(rB[p]) && a.fast_ok_c);
     }
 
     for (int region = 0; region < 2; ++region) {
@@ -441,8 +422,8 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long tile0,
                         my_steps += (unsigned long long)n;
                     } else {
                         PixelState ps{sx[p], sl[p], valid[p]};
-                        const bool dead = acc ? careful_steps<true>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps)
-                                              : careful_steps<false>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps);
+                        const bool dead = acc ? careful_steps<true>(&ps, rA, rB[p], rC, sel, wrap, s, n, &my_steps)
+                                              : careful_steps<false>(&ps, rA, rB[p], rC, sel, wrap, s, n, &my_steps);
                         x[p] = ps.x;
                         lyap[p] = ps.lyap;
                         valid[p] = ps.valid;
@@ -492,8 +473,8 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long tile0,
                     my_steps += (unsigned long long)n;
                 } else {
                     PixelState ps{sx[p], sl[p], valid[p]};
-                    const bool dead = acc ? careful_steps<true>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps)
-                                          : careful_steps<false>(&ps, rA[p], rB[p], rC, sel, wrap, s, n, &my_steps);
+                    const bool dead = acc ? careful_steps<true>(&ps, rA, rB[p], rC, sel, wrap, s, n, &my_steps)
+                                          : careful_steps<false>(&ps, rA, rB[p], rC, sel, wrap, s, n, &my_steps);
                     x[p] = ps.x;
                     lyap[p] = ps.lyap;
                     valid[p] = ps.valid;
@@ -513,42 +494,12 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long tile0,
         if (!done[p]) lam[p] = valid[p] > 0 ? __ddiv_rn(lyap[p], __dmul_rn((double)valid[p], LYAP_LN2)) : -5.0;
     }
 
-    // stores: each warp's 32*P consecutive values go through the warp's own staging row in shared memory, so that every
-    // lane writes 16 bytes and a store instruction covers consecutive 512-byte runs whatever P is (no block-wide barrier:
-    // warps stay out of step with each other); a ragged last tile or a misaligned output pointer takes plain stores
-    const bool full_tile = tile0 + 32 * P <= a.n_pixels;
-    if (out64) {
-        if (full_tile && ((reinterpret_cast<uintptr_t>(out64 + tile0) & 15) == 0)) {
-            __syncwarp();   // the row is free (this warp's reads of the previous tile are done)
+    if (!inside) return;
+    const long long at = row * a.width + col;
 #pragma unroll
-            for (int p = 0; p < P; ++p) stage[lane * P + p] = lam[p];
-            __syncwarp();
-            double2* dst = reinterpret_cast<double2*>(out64 + tile0);
-            const double2* src = reinterpret_cast<const double2*>(stage);
-#pragma unroll
-            for (int i = lane; i < 16 * P; i += 32) dst[i] = src[i];
-        } else {
-#pragma unroll
-            for (int p = 0; p < P; ++p)
-                if (idx0 + p < a.n_pixels) out64[idx0 + p] = lam[p];
-        }
-    }
-    if (out32) {
-        if (full_tile && ((reinterpret_cast<uintptr_t>(out32 + tile0) & 15) == 0)) {
-            float* stage32 = reinterpret_cast<float*>(stage);
-            __syncwarp();
-#pragma unroll
-            for (int p = 0; p < P; ++p) stage32[lane * P + p] = (float)lam[p];
-            __syncwarp();
-            float4* dst = reinterpret_cast<float4*>(out32 + tile0);
-            const float4* src = reinterpret_cast<const float4*>(stage32);
-#pragma unroll
-            for (int i = lane; i < 8 * P; i += 32) dst[i] = src[i];
-        } else {
-#pragma unroll
-            for (int p = 0; p < P; ++p)
-                if (idx0 + p < a.n_pixels) out32[idx0 + p] = (float)lam[p];
-        }
+    for (int p = 0; p < P; ++p) {
+        if (out64) out64[at + (long long)p * a.width] = lam[p];
+        if (out32) out32[at + (long long)p * a.width] = (float)lam[p];
     }
 }
 
@@ -580,23 +531,40 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
     // then the rest of the frame in tiles of 32 pixels; a block's tiles go round its four schedulers (a warp's scheduler is
     // warp % 4), and a warp that is done takes its scheduler's next tile from a counter in shared memory.  Warps whose orbits
     // leave (0,1) early so take more tiles, and the small ones at the end fill what the wide ones leave ragged: a scheduler's
-    // time is its pixels times a constant whatever its warps' shapes (2200 steps: 147 / 245 / 350 / 456 us for 1 / 2 / 3 / 4
-    // warps of 3 pixels a thread, 58 / 93 / 123 / 158 us for 1 / 2 / 3 / 4 of one).  With one counter a block the first
+    // time is its pixels times a constant whatever its warps' shapes (2200 steps: 103 / 168 / 238 / 312 us for 1 / 2 / 3 / 4
+    // warps of 2 pixels a thread, 58 / 93 / 123 / 158 us for 1 / 2 / 3 / 4 of one).  With one counter a block the first
     // scheduler to be done takes all small tiles of a frame of one round: 512 x 512 in 0.301 instead of 0.287 ms.
     __shared__ unsigned next_unit[4];   // the first units are taken as unit == warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < 4) next_unit[threadIdx.x] = THREADS / 32 + threadIdx.x;
     __syncthreads();   // the counters, and both tables, which are read across warps from the first logarithm on
+    // Positions are the columns of the rows in groups of P, group by group; a wide tile is 32 consecutive positions.  The
+    // small tiles go over the positions that are left, for each of the P rows in turn, and then over the rows behind the
+    // last whole group.
+    const long long rows = a.n_pixels / a.width, positions = rows / P * a.width;
+    const long long first = a.wide_tiles * 32, left = positions - first;
+    const long long narrow_pixels = a.n_pixels - first * P;
     const long long wide_of_block = a.wide_tiles > blockIdx.x ? (a.wide_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
-    double* stage = reinterpret_cast<double*>(smem_raw + kExactSmemBytes) + warp * (32 * P);
     for (unsigned unit = warp;;) {
         if (unit < wide_of_block) {
-            const long long tile = (long long)unit * gridDim.x + blockIdx.x;
-            exact_tile<P, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, tile * (32LL * P), out64, out32, stage, lane_off, my_steps);
+            const long long q = ((long long)unit * gridDim.x + blockIdx.x) * 32 + lane, group = q / a.width;
+            exact_tile<P, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, group * P, (int)(q - group * a.width), true, out64, out32, lane_off,
+                                                                my_steps);
         } else {
-            const long long at = a.wide_tiles * (32LL * P) + ((unit - wide_of_block) * gridDim.x + blockIdx.x) * 32;
-            if (at >= a.n_pixels) break;
-            exact_tile<1, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, at, out64, out32, stage, lane_off, my_steps);
+            const long long tile = ((unit - wide_of_block) * gridDim.x + blockIdx.x) * 32;
+            if (tile >= narrow_pixels) break;
+            const long long m = tile + lane;
+            long long row, col;
+            if (m < left * P) {
+                const long long p = m / left, q = first + (m - p * left);
+                row = q / a.width * P + p;
+                col = q % a.width;
+            } else {
+                const long long k = m - left * P;
+                row = rows / P * P + k / a.width;
+                col = k % a.width;
+            }
+            exact_tile<1, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, row, (int)col, m < narrow_pixels, out64, out32, lane_off, my_steps);
         }
         if (lane == 0) unit = atomicAdd(&next_unit[warp & 3], 4u);
         unit = __shfl_sync(0xFFFFFFFFu, unit, 0);

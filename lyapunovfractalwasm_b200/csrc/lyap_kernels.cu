@@ -6,6 +6,7 @@
 //   k_colorize       box mean + palette + RGBA store  (web/fractal_renderer.js:283-311,207-281,191-198)
 //
 // Build with -fmad=false: the exact kernels may only fuse where an fma is written out.
+#include <algorithm>
 #include <cfloat>
 #include <math_constants.h>
 #include <cstdint>
@@ -19,13 +20,18 @@
 
 namespace lyap {
 
-constexpr int kExactThreads = 512, kExactPixels = 3;   // measured best shape of the wide tiles on large frames
+// The wide tiles' shape.  2048 x 2048 of "AABAB" 200 + 2000 / "BBBBBBAAAAAA" 500 + 4000, frame 0 of the zoom (a third of its
+// orbits end) and the 800 x 800 page: 2 pixels a thread 7.92 / 15.75 / 4.48 / 0.676 ms, 3 pixels 7.90 / 15.96 / 4.66 / 0.716,
+// 3 pixels side by side in a row 7.84 / 15.80 / 4.90 / 0.705 (128 registers and a few spilled); 4 of 384 threads 8.00 / 16.9.
+// The generic kernel picks a straight-line body every two steps for all of a thread's pixels: 3 pixels 1.02 ms, 2 pixels 1.05
+// (1277 x 719, 37 letters, 100 + 1000).
+constexpr int kExactThreads = 512, kExactPixels = 2, kGenericPixels = 3;
 
 template <bool HAS_C>
 static cudaError_t launch_exact_generic(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                         unsigned grid, cudaStream_t st) {
-    auto kern = k_lambda_exact<kExactPixels, kExactThreads, HAS_C, 2>;
-    constexpr size_t smem = exact_smem_bytes(kExactThreads, kExactPixels);
+    auto kern = k_lambda_exact<kGenericPixels, kExactThreads, HAS_C, 2>;
+    constexpr size_t smem = kExactSmemBytes;
     // the attribute is per device and cheap to set; doing it on every launch keeps this thread- and device-safe
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -44,24 +50,32 @@ static int spec_mode() {
     return (jit < 0 ? 0 : (jit > 2 ? 2 : jit)) | (pre ? kSpecUsePrebuilt : 0);
 }
 
+// Deals a launch out for wide tiles of `pixels` a thread: whole rounds of them over the device's schedulers (4 an SM); 2 to 5
+// tiles of 32 pixels a scheduler are left to even out the end, and what is left of the rows' groups.  Returns the grid: the
+// shared tables allow one CTA per SM.
+static unsigned deal_exact(LambdaArgs* a, int pixels, int sm_count) {
+    const long long wide_px = 32LL * pixels, schedulers = 4LL * sm_count;
+    const long long rounds = std::min((a->n_pixels - 64 * schedulers) / (wide_px * schedulers),
+                                      a->n_pixels / a->width / pixels * a->width / (32 * schedulers));
+    a->wide_tiles = rounds > 0 ? rounds * schedulers : 0;
+    const long long warp_tiles = a->wide_tiles + (a->n_pixels - a->wide_tiles * wide_px + 31) / 32;
+    return (unsigned)std::min<long long>(warp_tiles, sm_count);
+}
+
 cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* out32, unsigned long long* steps,
                                 int sm_count, cudaStream_t st) {
     if (args.n_pixels <= 0) return cudaSuccess;
     LambdaArgs a = args;
+    // a periodic sequence can run an instance of this kernel made for its patterns
+    unsigned grid = deal_exact(&a, kExactPixels, sm_count);
+    bool launched = false;
+    const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads, kExactSmemBytes,
+                                             spec_mode(), &launched);
+    if (e != cudaSuccess || launched) return e;
     bool has_c = false;
     const int words = a.acc_word0 + (a.iterations > 0 ? min(a.acc_wrap, (a.iterations - 1) / kStepsPerWord + 1) : 0);
     for (int i = 0; i < words; ++i) has_c = has_c || (a.sel[i] & 0xAAAAAAAAu);
-    // wide tiles in whole rounds over the device's schedulers (4 an SM); 2 to 5 tiles of 32 pixels a scheduler are left to
-    // even out the end
-    const long long wide_px = 32LL * kExactPixels, schedulers = 4LL * sm_count;
-    a.wide_tiles = a.n_pixels > 64 * schedulers ? (a.n_pixels - 64 * schedulers) / (wide_px * schedulers) * schedulers : 0;
-    const long long warp_tiles = a.wide_tiles + (a.n_pixels - a.wide_tiles * wide_px + 31) / 32;
-    const unsigned grid = (unsigned)(warp_tiles < sm_count ? warp_tiles : sm_count);   // the shared tables allow one CTA per SM
-    // a periodic sequence can run an instance of this kernel made for its patterns
-    bool launched = false;
-    const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads,
-                                             exact_smem_bytes(kExactThreads, kExactPixels), spec_mode(), &launched);
-    if (e != cudaSuccess || launched) return e;
+    grid = deal_exact(&a, kGenericPixels, sm_count);
     return has_c ? launch_exact_generic<true>(a, out64, out32, steps, grid, st)
                  : launch_exact_generic<false>(a, out64, out32, steps, grid, st);
 }

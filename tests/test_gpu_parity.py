@@ -141,28 +141,25 @@ def test_ragged_shapes(engine, port, shape):
     assert same_bits(r["norm"], norm) and np.array_equal(r["rgba"], port.colorize(norm, 0))
 
 
-# pixels of one scheduler's tile of 32, and of its wide tile of 96, on a part of 148 multiprocessors with 4 schedulers each
-TILES, WIDE = 592 * 32, 592 * 96
-
-
-@pytest.mark.parametrize("pixels", [31, 33, 16 * 32 * 148 + 1, 2 * TILES + WIDE - 1, 2 * TILES + WIDE, 2 * TILES + WIDE + 1,
-                                    5 * TILES + WIDE + 17, 2 * TILES + 5 * WIDE + 32 * 7 + 5])
+# One round of wide tiles over a part of 148 multiprocessors with 4 schedulers each is 592 x 64 = 37888 pixels in pairs of
+# rows; at least as many are left for tiles of 32.
+@pytest.mark.parametrize("shape", [(31, 1), (33, 1), (1, 33), (75777, 1), (1, 75779), (37887, 2), (37888, 2), (25259, 3), (7, 20011),
+                                   (12629, 6), (613, 331)], ids=lambda s: "%dx%d" % s)
 @pytest.mark.parametrize("path", ["prebuilt", "generic"])
-def test_every_tile_of_a_launch_is_walked_once(engine, port, kernel_path, path, pixels):
-    """Frames of a few rounds of warp-tiles: all 32-pixel tiles, the first wide ones, a ragged last tile.  One row (and its
-    transpose's one column) has every pixel on another tile edge; the step count shows a tile that is walked twice."""
+def test_every_tile_of_a_launch_is_walked_once(engine, port, kernel_path, path, shape):
+    """Frames of less than a round of wide tiles and of a few, with rows and positions left over; the step count shows a
+    tile that is walked twice."""
     kernel_path(path)
-    for w, h in ((pixels, 1), (1, pixels)):
-        kw = dict(min_x=2.5, max_x=4.1, min_y=2.5, max_y=4.1, width=w, height=h, sequence="AB", iterations=40, warmup=8)
-        if h == 1:
-            kw.update(max_y=2.5 + 1e-9)
-        else:
-            kw.update(max_x=2.5 + 1e-9)
-        p = L.make_params(**kw)
-        r = engine.render(p, want=("lambda", "lambda32"))
-        lam, steps = oracle_rows(port, kw)
-        assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps, (w, h)
-        assert np.array_equal(r["lambda32"].view(np.uint32), lam.astype(np.float32).view(np.uint32))
+    w, h = shape
+    kw = dict(min_x=2.5, max_x=4.1, min_y=2.5, max_y=4.1, width=w, height=h, sequence="AB", iterations=40, warmup=8)
+    if h == 1:
+        kw.update(max_y=2.5 + 1e-9)
+    if w == 1:
+        kw.update(max_x=2.5 + 1e-9)
+    r = engine.render(L.make_params(**kw), want=("lambda", "lambda32"))
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps
+    assert np.array_equal(r["lambda32"].view(np.uint32), lam.astype(np.float32).view(np.uint32))
 
 
 @pytest.mark.parametrize("kw", [
