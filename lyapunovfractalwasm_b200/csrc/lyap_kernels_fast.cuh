@@ -160,18 +160,51 @@ __device__ __forceinline__ void fast_mode_steps(typename FL::real (&x)[P], typen
     }
 }
 
+// Below kFallen, 1 - 2x and 1 - x round to 1 and r - 2rx to r: a step is x <- r*x and its derivative the parameter itself.
+constexpr double kFallen = 0x1p-60;
+static __device__ __noinline__ double log_of(double d) { return lyap_log_tab(d, g_lyap_logtab, 1); }
+
 // fast_careful_chunk for steps [first, first + n) of a region whose selector words start at `sel`.
+// An orbit that runs down to zero (rA*rB < 1: a whole region of a frame over [0,4]^2 does, each orbit at another step) spends
+// most of them below kFallen, where the logarithm of a step's derivative is one of at most three taken beforehand: the
+// same sums, without a table look-up and a polynomial a step.  2048 x 1024 over [0.01,4]^2, "ABAAB" 120 + 1200: fused
+// fp64 4.97 -> 2.32 ms, on the exact orbit 3.60 -> 1.93 (without exits 0.69 and 0.90, as before).
 template <typename FL, bool ACC>
 __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                 typename FL::real rC, const unsigned* sel, int wrap, int first, int n,
                                                 unsigned long long* steps) {
-    bool dead = false;
+    using T = typename FL::real;
+    bool dead = false, logs = false;
+    double zA = 0.0, zB = 0.0, zC = 0.0;
     int j = first;
     const int end = first + n;
     while (j < end && !dead) {
         const int in_word = j & (kStepsPerWord - 1);
         const int m = min(kStepsPerWord - in_word, end - j);
-        dead = fast_careful_chunk<FL, ACC>(ps, rA, rB, rC, sel[(j / kStepsPerWord) % wrap] >> (2 * in_word), m, steps);
+        unsigned word = sel[(j / kStepsPerWord) % wrap] >> (2 * in_word);
+        int k = 0;
+        if (sizeof(T) == 8 && ps->x < (T)kFallen) {   // fp32 orbits are at zero too soon for it to pay
+            if (ACC && !logs) {
+                zA = log_of((double)rA);
+                zB = log_of((double)rB);
+                zC = log_of((double)rC);
+                logs = true;
+            }
+            T x = ps->x;
+            double extra = ps->extra;
+            for (; k < m && !dead && x < (T)kFallen; ++k, word >>= 2) {
+                const unsigned code = word & 3u;
+                if (code == 2u && !(rC > (T)0)) break;   // a third parameter that is no ordinary one
+                x = FastTraits<T>::mul(code == 0 ? rA : (code == 1 ? rB : rC), x);
+                if (ACC) extra = __dadd_rn(extra, code == 0 ? zA : (code == 1 ? zB : zC));
+                dead = !(x > (T)0);
+            }
+            if (ACC) ps->valid += k;
+            *steps += (unsigned long long)k;
+            ps->x = x;
+            ps->extra = extra;
+        }
+        if (k < m && !dead) dead = fast_careful_chunk<FL, ACC>(ps, rA, rB, rC, word, m - k, steps);
         j += m;
     }
     return dead;
@@ -481,8 +514,8 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                         prod[p] = sp[p];
                         FastPixel<T> ps{kSign * sx[p], extra[p], valid[p]};
                         const bool dead =
-                            acc ? fast_careful_chunk<FL, true>(&ps, rA[p], rB[p], rC[p], word, n, &my_steps)
-                                : fast_careful_chunk<FL, false>(&ps, rA[p], rB[p], rC[p], word, n, &my_steps);
+                            acc ? fast_careful_steps<FL, true>(&ps, rA[p], rB[p], rC[p], a.sel + word0, wrap, c * kStepsPerWord, n, &my_steps)
+                                : fast_careful_steps<FL, false>(&ps, rA[p], rB[p], rC[p], a.sel + word0, wrap, c * kStepsPerWord, n, &my_steps);
                         x[p] = kSign * ps.x;
                         extra[p] = ps.extra;
                         valid[p] = ps.valid;

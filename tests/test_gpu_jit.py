@@ -213,3 +213,22 @@ def test_packed_fp32_step_is_the_one_wide_step(engine, kernel_path, iterations):
         got[path] = engine.compute_fractal(L.make_params(**kw, mode=L.MODE_FAST_FP32))
         assert np.max(np.abs(got[path] - want)) < 3e-7 / smallest / np.log(2.0) + 1e-6, path   # + the products' roundings
     assert np.max(np.abs(got["jit"] - got["generic"])) < 2e-6
+
+
+@pytest.mark.parametrize("kw", [
+    dict(sequence="AB", max_x=1.1, max_y=1.1), dict(sequence="ABAAB", max_x=4.0, max_y=0.3), dict(sequence="AB" * 20 + "B", max_x=0.9, max_y=0.9),
+    dict(sequence="ABC", max_x=1.0, max_y=1.0, c=0.3), dict(sequence="AABBC", max_x=0.5, max_y=0.5, c=-1.0),
+], ids=lambda kw: "%s_%s" % (kw["sequence"][:6], kw.get("c")))
+@pytest.mark.parametrize("path", ["jit", "generic"])
+def test_fast_modes_on_orbits_that_run_down_to_zero(engine, port, kernel_path, path, kw):
+    """Exits by underflow in the fast fp64 modes: the executed steps are the exact mode's on its own orbit, and the sums
+    of up to 1300 logarithms below 10 in magnitude differ from its by roundings: 1300 * 1300 * 10 * 2^-53 / 1300 < 2e-12 a step."""
+    kernel_path(path)
+    kw = dict(dict(min_x=0.003, min_y=0.002, width=97, height=41, iterations=1300, warmup=150), **kw)
+    want, steps = oracle(port, kw)
+    r = engine.render(L.make_params(**kw, mode=L.MODE_FAST_FP64_ORBIT), want=("lambda",))
+    assert r["stats"].executed_steps == steps
+    assert np.max(np.abs(r["lambda"] - want)) < 2e-12
+    # the fused orbit rounds otherwise: an orbit may reach zero a step sooner or later, which moves a mean of n >= 1 terms
+    f = engine.compute_fractal(L.make_params(**kw, mode=L.MODE_FAST_FP64))
+    assert np.array_equal(f == -5.0, want == -5.0) and np.median(np.abs(f - want)) < 2e-12
