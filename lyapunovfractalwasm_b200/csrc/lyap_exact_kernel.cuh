@@ -384,20 +384,14 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
                     sx[p] = x[p];
                     sl[p] = lyap[p];
                 }
-                if (left >= CS) {             // CB whole periods, straight-line, REP times
+                if (left >= CB * BS) {        // CB whole periods, straight-line, REP times (or once)
 #pragma unroll 1
-                    for (int rep = 0; rep < REP; ++rep) {
+                    for (int rep = n / (CB * BS); rep > 0; --rep) {
 #pragma unroll
                         for (int b = 0; b < CB; ++b) {
                             if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
                             else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
                         }
-                    }
-                } else if (left >= CB * BS) { // one straight-line block
-#pragma unroll
-                    for (int b = 0; b < CB; ++b) {
-                        if (acc) period_block<P, true, KG, ACC_PATS>(x, lyap, rA, rB, rC, lane_off);
-                        else period_block<P, false, KG, WU_PATS>(x, lyap, rA, rB, rC, lane_off);
                     }
                 } else if (left >= BS) {      // the last few whole periods
 #pragma unroll 1
