@@ -57,8 +57,9 @@ def generate_jit_source():
         text = open(os.path.join(CSRC, name)).read()
         var = "kSrc_" + name.replace(".", "_")
         out.append("static const char %s[] =" % var)
-        for i in range(0, len(text), 8000):      # string literals are concatenated; keep each piece small
-            out.append('R"LYAPSRC(' + text[i:i + 8000] + ')LYAPSRC"')
+        size = -(-len(text) // -(-len(text) // 8000))   # string literals are concatenated; small pieces of one size
+        for i in range(0, len(text), size):
+            out.append('R"LYAPSRC(' + text[i:i + size] + ')LYAPSRC"')
         out.append(";")
     new = "\n".join(out) + "\n"
     if not os.path.exists(JIT_INC) or open(JIT_INC).read() != new:

@@ -93,8 +93,9 @@ __device__ __noinline__ bool careful_chunk(PixelState* ps, double rA, double rB,
 // register pair where fma(-2, x, 1) reads two, its second constant being one: the lambda kernel is bound by register reads
 // (a 64-bit pair a cycle and scheduler: two-operand fp64 instructions alone use them up, measured 1.98 cycles each, 2.96
 // with three distinct registers), and this one read fewer took 4096 x 2048 pixels of
-// "AABAB" 200 + 2000 from 16.11 to 15.73 ms.  What remains is the look-ups: two 16-byte loads a logarithm keep the SM's one
-// shared-memory data pipe busy for 32 of the 34 cycles that a scheduler now takes for a pixel and step.
+// "AABAB" 200 + 2000 from 16.11 to 15.73 ms.  Together the fp64 pipe (77 % busy on
+// the 4096^2 frame), the shared-memory data pipe (80 %, two 16-byte look-ups a logarithm) and the register reads of the seven
+// other instructions leave no gap that a change of one of them would fill.
 __device__ __forceinline__ double half_derivative(double r, double x) { return __dmul_rn(r, fabs(__dsub_rn(0.5, x))); }
 
 // Constants of the log core in constant memory: fp64 instructions take them as constant-bank
