@@ -161,7 +161,9 @@ __device__ __forceinline__ void fast_mode_steps(typename FL::real (&x)[P], typen
 }
 
 // Below kFallen, 1 - 2x and 1 - x round to 1 and r - 2rx to r: a step is x <- r*x and its derivative the parameter itself.
-constexpr double kFallen = 0x1p-60;
+// A parameter of at most kFallenParam takes such an x to less than 1/2, so that zero is the only way out of (0,1); the
+// comparison is false for NaN, whose derivative is no term of the sum, and for infinity.
+constexpr double kFallen = 0x1p-60, kFallenParam = 0x1p59;
 static __device__ __noinline__ double log_of(double d) { return lyap_log_tab(d, g_lyap_logtab, 1); }
 
 // fast_careful_chunk for steps [first, first + n) of a region whose selector words start at `sel`.
@@ -174,6 +176,8 @@ __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps
                                                 typename FL::real rC, const unsigned* sel, int wrap, int first, int n,
                                                 unsigned long long* steps) {
     using T = typename FL::real;
+    // fp32 orbits are at zero too soon for it to pay
+    const bool may_fall = sizeof(T) == 8 && rA <= (T)kFallenParam && rB <= (T)kFallenParam;
     bool dead = false, logs = false;
     double zA = 0.0, zB = 0.0, zC = 0.0;
     int j = first;
@@ -183,7 +187,7 @@ __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps
         const int m = min(kStepsPerWord - in_word, end - j);
         unsigned word = sel[(j / kStepsPerWord) % wrap] >> (2 * in_word);
         int k = 0;
-        if (sizeof(T) == 8 && ps->x < (T)kFallen) {   // fp32 orbits are at zero too soon for it to pay
+        if (may_fall && ps->x < (T)kFallen) {
             if (ACC && !logs) {
                 zA = log_of((double)rA);
                 zB = log_of((double)rB);
@@ -194,7 +198,7 @@ __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps
             double extra = ps->extra;
             for (; k < m && !dead && x < (T)kFallen; ++k, word >>= 2) {
                 const unsigned code = word & 3u;
-                if (code == 2u && !(rC > (T)0)) break;   // a third parameter that is no ordinary one
+                if (code == 2u && !(rC > (T)0 && rC <= (T)kFallenParam)) break;
                 x = FastTraits<T>::mul(code == 0 ? rA : (code == 1 ? rB : rC), x);
                 if (ACC) extra = __dadd_rn(extra, code == 0 ? zA : (code == 1 ? zB : zC));
                 dead = !(x > (T)0);

@@ -36,6 +36,9 @@ class Port:
         L.oracle_lambda_rows.argtypes = [ctypes.c_double] * 4 + [ctypes.c_int] * 2 + [
             ctypes.c_char_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
             ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, c_double_p]
+        L.oracle_fused_lambda.restype = ctypes.c_uint64
+        L.oracle_fused_lambda.argtypes = [ctypes.c_double] * 4 + [ctypes.c_int] * 2 + [
+            ctypes.c_char_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_int, c_double_p]
         L.oracle_minmax.argtypes = [c_double_p, ctypes.c_uint64, c_double_p, c_double_p]
         L.oracle_normalize_with.argtypes = [c_double_p, ctypes.c_uint64, ctypes.c_double, ctypes.c_double,
                                             c_double_p]
@@ -60,6 +63,14 @@ class Port:
         steps = self.lib.oracle_lambda_rows(min_x, max_x, min_y, max_y, width, height, seq, len(seq), iterations,
                                             warmup, 0 if c is None else 1, 0.0 if c is None else c, y0, y1,
                                             row_stride, _dp(out))
+        return out, int(steps)
+
+    def fused_lambda(self, min_x, max_x, min_y, max_y, width, height, sequence, iterations, warmup, c=None, single=False):
+        """The whole frame in the fused fp64 (single: fp32) step, logarithms summed in extended precision -> (array, steps)."""
+        out = np.empty((height, width), dtype=np.float64)
+        seq = sequence.encode("latin-1")
+        steps = self.lib.oracle_fused_lambda(min_x, max_x, min_y, max_y, width, height, seq, len(seq), iterations, warmup,
+                                             0 if c is None else 1, 0.0 if c is None else c, 1 if single else 0, _dp(out))
         return out, int(steps)
 
     def minmax(self, v):

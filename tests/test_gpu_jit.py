@@ -229,6 +229,28 @@ def test_fast_modes_on_orbits_that_run_down_to_zero(engine, port, kernel_path, p
     r = engine.render(L.make_params(**kw, mode=L.MODE_FAST_FP64_ORBIT), want=("lambda",))
     assert r["stats"].executed_steps == steps
     assert np.max(np.abs(r["lambda"] - want)) < 2e-12
-    # the fused orbit rounds otherwise: an orbit may reach zero a step sooner or later, which moves a mean of n >= 1 terms
-    f = engine.compute_fractal(L.make_params(**kw, mode=L.MODE_FAST_FP64))
-    assert np.array_equal(f == -5.0, want == -5.0) and np.median(np.abs(f - want)) < 2e-12
+    # the fused orbit rounds otherwise: it has a restatement of its own
+    want, steps = port.fused_lambda(**kw)
+    r = engine.render(L.make_params(**kw, mode=L.MODE_FAST_FP64), want=("lambda",))
+    assert r["stats"].executed_steps == steps
+    assert np.max(np.abs(r["lambda"] - want)) < 2e-12
+
+
+@pytest.mark.parametrize("kw", [
+    dict(sequence="A" * 40 + "C", c=1e30), dict(sequence="A" * 15 + "C", c=1e30), dict(sequence="A" * 15 + "C", c=2.0 ** 61),
+    dict(sequence="A" * 15 + "C", c=np.inf), dict(sequence="A" * 15 + "C", c=np.nan), dict(sequence="A" * 15 + "C", c=2.0 ** 59),
+    dict(sequence="A" * 20 + "B", max_y=1e30), dict(sequence="A" * 15 + "B", max_y=2.0 ** 60), dict(sequence="A" * 15 + "B", max_y=np.inf),
+    dict(sequence="A" * 20 + "B", height=1), dict(sequence="B" * 20 + "A", width=1), dict(sequence="A" * 15 + "C", c=1e30, width=1, height=1),
+], ids=lambda kw: "_".join("%s" % (v,) for v in kw.values()))
+@pytest.mark.parametrize("path", ["jit", "generic"])
+def test_fast_modes_on_falls_that_a_large_or_undefined_parameter_ends(engine, port, kernel_path, path, kw):
+    """Orbits below 2^-60 when a parameter beyond 2^59 (out of (0,1) in one step), an infinite one or NaN (a frame of one row
+    or column has such a one: 0 * inf) comes up, in warm-up and in accumulation: the exits and terms of the step-by-step rules.
+    200 logarithms of at most 709 in magnitude: 200 * 709 * 2^-53 / ln 2 = 2.3e-11 of rounding in a mean."""
+    kernel_path(path)
+    for warmup in (0, 15, 16, 21, 47):
+        k = dict(dict(min_x=0.04, max_x=0.3, min_y=0.05, max_y=0.3, width=19, height=7, iterations=200, warmup=warmup), **kw)
+        for mode, (want, steps) in ((L.MODE_FAST_FP64_ORBIT, oracle(port, k)), (L.MODE_FAST_FP64, port.fused_lambda(**k))):
+            r = engine.render(L.make_params(**k, mode=mode), want=("lambda",))
+            assert r["stats"].executed_steps == steps, (mode, warmup)
+            np.testing.assert_allclose(r["lambda"], want, rtol=0.0, atol=2.4e-11)
