@@ -88,8 +88,8 @@ constexpr int kMinmaxThreads = 256;
 
 __device__ __forceinline__ void minmax_take(double v, double& lo, double& hi) {
     if (v > -4.0 && v <= DBL_MAX) {     // :116
-        lo = v < lo ? v : lo;          // neither is NaN: a comparison and a select, where fmin takes care of NaN
-        hi = v > hi ? v : hi;
+        lo = fmin(lo, v);              // of zeros the negative one, whichever comes first: a comparison and a select would
+        hi = fmax(hi, v);              // make the sign depend on how the values are dealt out
     }
 }
 

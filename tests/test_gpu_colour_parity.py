@@ -138,3 +138,26 @@ def test_normalise_edges_and_special_values(engine, port, n):
             at = rng.integers(0, n, size=max(1, n // 5))
             values[at] = rng.choice([-5.0, -4.0, -3.9999999, np.nan, np.inf, -np.inf, 0.0, 1e-310, -3.0, 1.2], size=at.size)
         assert same_bits(engine.normalize_data(values), port.normalize(values)), special
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 64, 4097, 700001])
+def test_minmax_of_zeros_does_not_depend_on_their_order(engine, n):
+    """Where the extreme is zero, the minimum is -0 and the maximum +0 if there is one, wherever it stands and however the
+    array is aligned (a thread's loads, its block and the last block each choose between two)."""
+    d_v, d_mm = engine.alloc(8 * (n + 1)), engine.alloc(16)
+    rng = np.random.default_rng(n)
+    for flip in (1.0, -1.0):
+        for offset in (0, 8):
+            for fill in (-1.0, 0.0, 1.0):
+                values = rng.permutation(np.where(np.arange(n) < max(2, n // 2), 0.0, fill))
+                at = np.flatnonzero(values == 0.0)
+                values[at] = flip * 0.0
+                values[rng.choice(at)] = -flip * 0.0
+                d_v.from_host(values, offset)
+                engine.minmax_device(d_v.ptr + offset, n, d_mm.ptr)
+                lo, hi = d_mm.to_host(np.float64)
+                assert lo == values.min() and hi == values.max()
+                assert lo != 0.0 or np.signbit(lo), (flip, offset, fill)
+                assert hi != 0.0 or not np.signbit(hi), (flip, offset, fill)
+    d_v.free()
+    d_mm.free()
