@@ -290,8 +290,9 @@ constexpr int kNormThreads = 256;
 struct ColourConsts {
     double invln2, ln2hi, ln2lo, exp_c[13], log_c2, log_c3, log_c4, klo_bias;
     double two_over_pi, pio2[3], sin_c[7], cos_c[7];
-    double pi, ninth, third2pi, third4pi, pal[5];   // pal: 0.8, 0.3, 0.9, 0.7, 0.6
+    double pi, third2pi, third4pi, pal[5];   // pal: 0.8, 0.3, 0.9, 0.7, 0.6
     double fifth, tenth, p95, y12;
+    double recip[10];                         // of a number of neighbours
 };
 static __constant__ ColourConsts c_col = {
     LYAP_INVLN2, LYAP_LN2HI, LYAP_LN2LO,
@@ -301,7 +302,8 @@ static __constant__ ColourConsts c_col = {
     LYAP_2OVERPI, {LYAP_PIO2_1, LYAP_PIO2_2, LYAP_PIO2_3},
     {LYAP_SIN_C0, LYAP_SIN_C1, LYAP_SIN_C2, LYAP_SIN_C3, LYAP_SIN_C4, LYAP_SIN_C5, LYAP_SIN_C6},
     {LYAP_COS_C0, LYAP_COS_C1, LYAP_COS_C2, LYAP_COS_C3, LYAP_COS_C4, LYAP_COS_C5, LYAP_COS_C6},
-    LYAP_PI, 1.0 / 9.0, 2.0 * LYAP_PI / 3.0, 4.0 * LYAP_PI / 3.0, {0.8, 0.3, 0.9, 0.7, 0.6}, 0.2, 0.1, 0.95, 1.2};
+    LYAP_PI, 2.0 * LYAP_PI / 3.0, 4.0 * LYAP_PI / 3.0, {0.8, 0.3, 0.9, 0.7, 0.6}, 0.2, 0.1, 0.95, 1.2,
+    {0.0, 1.0, 1.0 / 2.0, 1.0 / 3.0, 1.0 / 4.0, 1.0 / 5.0, 1.0 / 6.0, 1.0 / 7.0, 1.0 / 8.0, 1.0 / 9.0}};
 
 // lyap_exp for |x| <= 600: no special values, and the power of two goes in by adding to the exponent field (lyap_exp
 // multiplies by it: the same, as nothing leaves the normal range).  The integer is the low word of the shifted sum; a
@@ -418,6 +420,15 @@ cudaError_t launch_normalize(const double* v, unsigned long long n, const double
     return cudaGetLastError();
 }
 
+// A block for kernels whose threads each take a column of a strip of rows: the width dealt out evenly over as few blocks as
+// cover it, and as many strips on top of one another as there are threads left.  Whole warps of columns where a block has
+// one strip; in a narrower frame a warp goes on with the next strip's first columns.
+static dim3 column_block(int width, int threads) {
+    const long long blocks = ((long long)width + threads - 1) / threads;
+    const int columns = (int)((width + blocks - 1) / blocks);
+    return columns > threads / 2 ? dim3((unsigned)(columns + 31) / 32 * 32, 1) : dim3((unsigned)columns, (unsigned)(threads / columns));
+}
+
 // ---------------------------------------------------------------------------------------------
 // Colour stage: 3x3 mean (edge-aware, fixed summation order) -> palette -> clamped bytes, alpha 255.
 // ---------------------------------------------------------------------------------------------
@@ -495,8 +506,9 @@ __device__ __noinline__ unsigned palette_rgba(double t, int palette, const lyap_
     return clamp_u8(r) | (clamp_u8(g) << 8) | (clamp_u8(b) << 16) | 0xFF000000u;
 }
 
-// The palette for the t of a picture, 2^-300 <= t <= 1: palette_rgba's operations without special cases.  Sine and cosine of
-// one angle share their reduction and their two polynomials, and a channel's floor is one addition that rounds down.
+// The palette for the t of a picture, 0 <= t <= 1 (nebula: 2^-300 <= t): palette_rgba's operations without special cases.
+// Sine and cosine of one angle share their reduction and their two polynomials, and a channel's floor is one addition that
+// rounds down.
 __device__ __forceinline__ void sincos_plain(double x, double* sn, double* cs) {   // 0 <= x <= 24: lyap_sin, lyap_cos
     const double magic = 0x1.8p52;
     const double z = __fma_rn(x, c_col.two_over_pi, magic);
@@ -573,37 +585,13 @@ __device__ __forceinline__ unsigned palette_plain(double t, const lyap_logtab_en
 
 constexpr int kColorThreads = 256;
 
-// one pixel: 3x3 mean in the page's summation order, then the palette
-__device__ __noinline__ unsigned int colorize_one(const double* __restrict__ norm, long long idx, int width, long long rows,
-                                                     int rows_above, int rows_below, int palette, const lyap_logtab_entry* tab) {
-    const long long y = idx / width;
-    const int x = (int)(idx - y * width);
-    double sum = norm[idx];                       // :292
-    int count = 1;
-#pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
-        const long long ny = y + dy;
-        const bool row_ok = (ny >= 0 || rows_above) && (ny < rows || rows_below);
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-            if (dx == 0 && dy == 0) continue;
-            const int nx = x + dx;
-            if (row_ok && nx >= 0 && nx < width) {       // :301
-                sum = __dadd_rn(sum, norm[ny * width + nx]);
-                ++count;
-            }
-        }
-    }
-    const double t = __ddiv_rn(sum, (double)count);      // :307
-    return palette_rgba(t, palette, tab);
-}
-
-// One pixel from its 3 x 3 values (row by row): summed in the page's order, and divided by nine through the reciprocal:
-// with y = RN(1/9), q = RN(s*y) is within an ulp of s/9, and RN(q + y*(s - 9q)) is s/9 correctly rounded (Markstein 1990).
-// A mean below 2^-300 or above 1 goes the general way.
+// One pixel from its 3 x 3 values (row by row), `count` of them there: summed in the page's order, and divided through the
+// reciprocal: with y = RN(1/n), q = RN(s*y) is within an ulp of s/n, and RN(q + y*(s - nq)) is s/n correctly rounded
+// (Markstein 1990).  A mean above 1 goes the general way, one below 2^-300 where the palette takes its power: the others'
+// channels are multiples of I or functions of `mid`, 0 and 1 for any t below 2^-54.
 template <int PALETTE>
 __device__ __forceinline__ unsigned colorize_inner(const double (&above)[3], const double (&row)[3], const double (&below)[3],
-                                                   const lyap_logtab_entry* tab) {
+                                                   double count, double recip, const lyap_logtab_entry* tab) {
     double s = row[1];                                                                   // :292
 #pragma unroll
     for (int k = 0; k < 3; ++k) s = __dadd_rn(s, above[k]);
@@ -611,38 +599,41 @@ __device__ __forceinline__ unsigned colorize_inner(const double (&above)[3], con
     s = __dadd_rn(s, row[2]);
 #pragma unroll
     for (int k = 0; k < 3; ++k) s = __dadd_rn(s, below[k]);
-    const double ninth = c_col.ninth;
-    const double q = __dmul_rn(s, ninth);
-    const double t = __fma_rn(__fma_rn(-9.0, q, s), ninth, q);                           // :307
-    if (t >= 0x1p-300 && t <= 1.0) return palette_plain<PALETTE>(t, tab);
-    return palette_rgba(__ddiv_rn(s, 9.0), PALETTE, tab);
+    const double q = __dmul_rn(s, recip);
+    const double t = __fma_rn(__fma_rn(-count, q, s), recip, q);                         // :307
+    if (t >= (PALETTE == 1 ? 0x1p-300 : 0.0) && t <= 1.0) return palette_plain<PALETTE>(t, tab);
+    return palette_rgba(__ddiv_rn(s, count), PALETTE, tab);
 }
 
-// A block takes 256 columns of kColorRows rows, a thread one column: its rows' values and their left and right neighbours are
-// loaded once, side by side across the warp, and stay in registers for the pixels above and below.  Pixels at the frame's
-// edges go one by one.  The palette is a template parameter: its code is then straight-line.
+// A thread takes one column of kColorRows rows: its rows' values and their left and right neighbours are loaded once, side by
+// side across the warp, and stay in registers for the pixels above and below.  A block is up to 256 columns wide and, in a
+// narrow frame, as many strips high as fill it.  A warp with a pixel at the frame's edge loads -0 for a neighbour that is
+// not there, which leaves any sum as it is.  The palette is a template parameter: its code is then straight-line.
 // 3840 x 2160, aurora / solarflare (the cheapest palette): 95 / 85 us with nine loads behind tests a pixel, 66 / 55 us with
 // four pixels of a row to a thread (18 loads, but 32 bytes apart across the warp), 52 / 38 us as here; with the tests for
-// the rows that exist inside the strip's code, 64-bit and uniform, it was 82 / 68.
+// the rows that exist inside every strip's code, 64-bit and uniform, it was 82 / 68.
+// Solarflare, two million pixels in 32 / 8 columns: 31 / 32 us with nine loads a pixel, 117 / 432 in blocks of 256 columns of
+// one strip, 19 / 21 so.
 constexpr int kColorRows = 4;
 
 template <int PALETTE>
-__global__ void __launch_bounds__(kColorThreads)
+__global__ void __launch_bounds__(kColorThreads, 4)
 k_colorize(const double* __restrict__ norm, int width, long long rows, int rows_above, int rows_below,
            unsigned int* __restrict__ rgba) {
     __shared__ lyap_logtab_entry tab[LYAP_LOG_BINS];
     if (PALETTE == 1) {
-        for (int e = threadIdx.x; e < LYAP_LOG_BINS; e += kColorThreads) tab[e] = g_lyap_logtab[e];
+        for (int e = threadIdx.y * blockDim.x + threadIdx.x; e < LYAP_LOG_BINS; e += blockDim.x * blockDim.y) tab[e] = g_lyap_logtab[e];
         __syncthreads();
     }
-    const long long x = (long long)blockIdx.x * kColorThreads + threadIdx.x;
+    const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= width) return;
-    for (long long y0 = (long long)blockIdx.y * kColorRows; y0 < rows; y0 += (long long)gridDim.y * kColorRows) {
+    const long long step = (long long)gridDim.y * blockDim.y * kColorRows;
+    for (long long y0 = ((long long)blockIdx.y * blockDim.y + threadIdx.y) * kColorRows; y0 < rows; y0 += step) {
         const double* at = norm + (y0 - 1) * width + x;   // in the row above: read only if that exists
         const bool whole = (y0 > 0 || rows_above) && (y0 + kColorRows < rows || (y0 + kColorRows == rows && rows_below));
         unsigned int* out = rgba + y0 * width + x;
-        if (whole && x > 0 && x < width - 1) {
-            double v[kColorRows + 2][3];
+        double v[kColorRows + 2][3];
+        if (__all_sync(__activemask(), whole && x > 0 && x < width - 1)) {
 #pragma unroll
             for (int r = 0; r < kColorRows + 2; ++r) {
 #pragma unroll
@@ -651,12 +642,29 @@ k_colorize(const double* __restrict__ norm, int width, long long rows, int rows_
             }
 #pragma unroll
             for (int r = 0; r < kColorRows; ++r) {
-                *out = colorize_inner<PALETTE>(v[r], v[r + 1], v[r + 2], tab);
+                *out = colorize_inner<PALETTE>(v[r], v[r + 1], v[r + 2], 9.0, c_col.recip[9], tab);
                 out += width;
             }
-        } else {   // the frame's edges, and the last strip of a height that is not a multiple of kColorRows
-            for (long long y = y0; y < rows && y < y0 + kColorRows; ++y, out += width)
-                *out = colorize_one(norm, y * width + x, width, rows, rows_above, rows_below, PALETTE, tab);
+        } else {
+            const bool left = x > 0, right = x < width - 1;
+            const int there = (int)min(rows - y0, (long long)kColorRows + 1);             // own rows of the strip and below it
+            const int first = y0 > 0 || rows_above ? 0 : 1, last = there + (there <= kColorRows && rows_below ? 1 : 0);
+#pragma unroll
+            for (int r = 0; r < kColorRows + 2; ++r) {
+                const bool row = r >= first && r <= last;
+                v[r][0] = row && left ? at[-1] : -0.0;
+                v[r][1] = row ? at[0] : -0.0;
+                v[r][2] = row && right ? at[1] : -0.0;
+                at += width;
+            }
+            const int columns = 1 + left + right;
+#pragma unroll
+            for (int r = 0; r < kColorRows; ++r) {
+                if (r >= there) break;
+                const int count = columns * (1 + (r >= first) + (r + 2 <= last));
+                *out = colorize_inner<PALETTE>(v[r], v[r + 1], v[r + 2], (double)count, c_col.recip[count], tab);
+                out += width;
+            }
         }
     }
 }
@@ -665,8 +673,9 @@ cudaError_t launch_colorize(const double* norm, int width, long long rows, int r
                             int palette, unsigned char* rgba, int sm_count, cudaStream_t st) {
     const long long n = rows * (long long)width;
     if (n <= 0) return cudaSuccess;
-    const long long strips = (rows + kColorRows - 1) / kColorRows;
-    const dim3 grid((unsigned)((width + kColorThreads - 1LL) / kColorThreads), (unsigned)(strips < 65535 ? strips : 65535));
+    const dim3 block = column_block(width, kColorThreads);
+    const long long strips = (rows + kColorRows - 1) / kColorRows, high = (strips + block.y - 1) / block.y;
+    const dim3 grid((unsigned)((width + block.x - 1LL) / block.x), (unsigned)(high < 65535 ? high : 65535));
     auto kern = k_colorize<0>;
     switch (palette) {
         case 1: kern = k_colorize<1>; break;
@@ -677,7 +686,7 @@ cudaError_t launch_colorize(const double* norm, int width, long long rows, int r
         case 6: kern = k_colorize<6>; break;
         default: break;
     }
-    kern<<<grid, kColorThreads, 0, st>>>(norm, width, rows, rows_above, rows_below, reinterpret_cast<unsigned int*>(rgba));
+    kern<<<grid, block, 0, st>>>(norm, width, rows, rows_above, rows_below, reinterpret_cast<unsigned int*>(rgba));
     return cudaGetLastError();
 }
 

@@ -1,6 +1,7 @@
 """GPU tests of the C ABI's behaviour around the kernels: host entry points, device entry points per
 band, error statuses, the progress callback, fast modes within their stated tolerance."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -221,6 +222,32 @@ def test_glow_at_the_edges_of_its_tiles(engine, port, shape):
     w, h = shape
     rgba = np.random.default_rng(w * 1000 + h).integers(0, 256, size=(h, w, 4), dtype=np.uint8)
     assert np.array_equal(engine.glow(rgba), port.glow(rgba))
+
+
+def per_call(engine, call, repeat=10):
+    """Seconds a call, of `repeat` enqueued ones."""
+    call()
+    engine.sync()
+    t0 = time.perf_counter()
+    for _ in range(repeat):
+        call()
+    engine.sync()
+    return (time.perf_counter() - t0) / repeat
+
+
+@pytest.mark.parametrize("stage", ["colour"])
+@pytest.mark.parametrize("width,height", [(8, 131072), (32, 32768), (131072, 8)])
+def test_shape_of_a_picture_does_not_set_its_time(engine, width, height, stage):
+    """A million pixels in 8 and 32 columns, and in 8 rows, against 1024 x 1024: blocks that do not fill with such a picture's
+    columns took 4 to 15 times as long, full ones take 0.7 to 1.4 times."""
+    n = 1 << 20
+    norm, rgba = engine.alloc(8 * n), engine.alloc(4 * n)
+    norm.from_host(np.random.default_rng(3).uniform(size=n))
+    calls = {"colour": lambda w, h: engine.colorize_device(norm.ptr, w, h, 0, 0, 2, rgba.ptr)}
+    seconds, square = (per_call(engine, lambda: calls[stage](w, h)) for w, h in ((width, height), (1024, 1024)))
+    assert seconds < 3.0 * square + 10e-6
+    for b in (norm, rgba):
+        b.free()
 
 
 def test_render_frames_batch_equals_frame_by_frame(engine, port):

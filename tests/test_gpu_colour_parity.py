@@ -113,9 +113,11 @@ def test_config4_colour_stage_on_a_band_with_given_minmax(engine, port):
 SPECIAL = [0.0, -0.0, 1.0, 0.5, 1e-310, 2.0 ** -301, 2.0 ** -300, 1.0 + 2.0 ** -52, 3.0, -0.25, 100.0, np.nan]
 
 
-@pytest.mark.parametrize("shape", [(1, 5), (2, 4), (3, 6), (9, 7), (255, 9), (256, 4), (257, 5), (258, 12), (513, 6)])
+@pytest.mark.parametrize("shape", [(1, 5), (2, 4), (3, 6), (9, 7), (255, 9), (256, 4), (257, 5), (258, 12), (513, 6),
+                                   (1, 2049), (2, 1030), (3, 700), (7, 297), (32, 65), (33, 57), (127, 22), (128, 18), (129, 13)])
 def test_colour_kernel_edges_and_special_values(engine, port, shape):
-    """Every palette at widths around a block's 256 columns and heights around a strip's 4 rows; half of the frames carry
+    """Every palette at widths around a block's 256 columns, heights around a strip's 4 rows and, in narrow frames, around
+    the strips of a block; half of the frames carry
     values a picture has none of, which take the general palette code: bytes equal the oracle's."""
     w, h = shape
     rng = np.random.default_rng(w * 100 + h)
