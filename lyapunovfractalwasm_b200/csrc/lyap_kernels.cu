@@ -710,51 +710,91 @@ struct GlowArgs {
 // which leaves a sum that is not negative as it is.  1920 x 1080, all three draws: 303 us with an output a thread, its
 // taps behind tests and the canvas looked up per tap; 149 us so (fp64 alone: 69).  8 columns' outputs a thread with at
 // most 128 registers; without that limit 175 us, 6 outputs 155, 12 outputs 171.
+// Pictures of which a block's row or strip would be half empty have several to a block, once they have rows enough for all
+// SMs (the instance for one has the block's shape as a constant: 1920 x 1080 in 147 us, with the other 152).  Two million pixels
+// in 32 / 8 / 1 columns: 303 / 266 / 258 us with an output a thread, 546 / 1890 / 14160 in blocks of one row, 175 / 164 / 207 so.
 constexpr int kGlowRowOut = 9;                      // odd: 9 outputs a thread put the lanes' inputs in different banks
 constexpr int kGlowRowThreads = 96;                 // 32 threads a channel
-constexpr int kGlowRowPixels = 32 * kGlowRowOut;    // of one row, a block
 constexpr int kGlowColOut = 8, kGlowColThreads = 128;
+constexpr int kGlowTall = 2048;
 
-template <int R>
+// some_lanes: those of each channel's 32 that work on one row, if the block has several
+template <int R, bool kOneRow>
 __global__ void __launch_bounds__(kGlowRowThreads)
-k_glow_blur_rows(const __grid_constant__ GlowArgs g, const unsigned char* __restrict__ canvas, int width, int height,
+k_glow_blur_rows(const __grid_constant__ GlowArgs g, const unsigned char* __restrict__ canvas, int width, int height, int some_lanes,
                  double* __restrict__ tmp) {
-    constexpr int kIn = kGlowRowPixels + 2 * R;
+    extern __shared__ double in_all[];   // of each channel, of each row: the outputs' inputs and R more on either side
     __shared__ double unit[256];
-    __shared__ double in[3][kIn];
     for (int i = threadIdx.x; i < 256; i += kGlowRowThreads) unit[i] = __ddiv_rn((double)i, 255.0);
-    const long long x0 = (long long)blockIdx.x * kGlowRowPixels;
+    constexpr int kOut = kGlowRowOut;
+    const int lanes = kOneRow ? 32 : some_lanes, rows = 32 / lanes, columns = lanes * kOut, pitch = columns + 2 * R, inputs = rows * pitch;
+    const long long x0 = (long long)blockIdx.x * columns;
     const int channel = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int lane_row = lane / lanes, lane_column = (lane - lane_row * lanes) * kOut;
+    const bool idle = lane_row >= rows;   // 32 is no multiple of every number of lanes
+    double* in = in_all + channel * inputs;
     const long long plane = (long long)width * height;
-    for (long long y = blockIdx.y; y < height; y += gridDim.y) {
-        const uchar4* row = reinterpret_cast<const uchar4*>(canvas) + y * width;
+    for (long long y0 = (long long)blockIdx.y * rows; y0 < height; y0 += (long long)gridDim.y * rows) {
         __syncthreads();
-        for (int i = threadIdx.x; i < kIn; i += kGlowRowThreads) {
-            const long long x = x0 + i - R;
-            const bool inside = x >= 0 && x < width;
-            const uchar4 c = inside ? row[x] : make_uchar4(0, 0, 0, 0);   // unit[0] is 0
-            in[0][i] = unit[c.x];
-            in[1][i] = unit[c.y];
-            in[2][i] = unit[c.z];
+        for (int i = threadIdx.x; i < inputs; i += kGlowRowThreads) {
+            const int r = rows > 1 ? i / pitch : 0;
+            const long long x = x0 + (i - r * pitch) - R, y = y0 + r;
+            const bool inside = x >= 0 && x < width && y < height;
+            const uchar4 c = inside ? reinterpret_cast<const uchar4*>(canvas)[y * width + x] : make_uchar4(0, 0, 0, 0);   // unit[0] is 0
+            in_all[i] = unit[c.x];
+            in_all[i + inputs] = unit[c.y];
+            in_all[i + 2 * inputs] = unit[c.z];
         }
         __syncthreads();
-        double s[kGlowRowOut];
+        double s[kOut];
 #pragma unroll
-        for (int o = 0; o < kGlowRowOut; ++o) s[o] = 0.0;
-        const double* at = in[channel] + lane * kGlowRowOut;
+        for (int o = 0; o < kOut; ++o) s[o] = 0.0;
+        double* at = in + (idle ? 0 : lane_row * pitch + lane_column);
 #pragma unroll
-        for (int j = 0; j < kGlowRowOut + 2 * R; ++j) {
+        for (int j = 0; j < kOut + 2 * R; ++j) {
             const double v = at[j];
 #pragma unroll
-            for (int o = 0; o < kGlowRowOut; ++o)
+            for (int o = 0; o < kOut; ++o)
                 if (j >= o && j <= o + 2 * R) s[o] = __dadd_rn(s[o], __dmul_rn(g.w[j - o], v));
         }
         __syncthreads();   // all inputs are read: the outputs take their place, to be written in order
+        if (!idle) {
 #pragma unroll
-        for (int o = 0; o < kGlowRowOut; ++o) in[channel][lane * kGlowRowOut + o] = s[o];
+            for (int o = 0; o < kOut; ++o) at[o] = s[o];
+        }
         __syncwarp();      // a warp writes its own channel
-        double* out = tmp + channel * plane + y * width;
-        for (int i = lane; i < kGlowRowPixels && x0 + i < width; i += 32) out[x0 + i] = in[channel][i];
+        const int there = (int)min((long long)columns, width - x0), n = (int)min((long long)rows, height - y0) * there;
+        double* out = tmp + channel * plane + y0 * width + x0;   // several rows are whole ones
+        for (int i = lane; i < n; i += 32) {
+            const int r = rows > 1 ? i / there : 0;
+            out[i] = in[r * pitch + (i - r * there)];
+        }
+    }
+}
+
+// The rows' blur of a picture of at most kGlowNarrow columns: few taps are inside it, and a lane's outputs would be more than
+// it has.
+constexpr int kGlowNarrow = 8;
+template <int R>
+__global__ void __launch_bounds__(kGlowColThreads)
+k_glow_blur_rows_narrow(const __grid_constant__ GlowArgs g, const unsigned char* __restrict__ canvas, int width, long long n,
+                        double* __restrict__ tmp) {
+    __shared__ double unit[256];
+    for (int i = threadIdx.x; i < 256; i += kGlowColThreads) unit[i] = __ddiv_rn((double)i, 255.0);
+    __syncthreads();
+    for (long long i = (long long)blockIdx.x * kGlowColThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kGlowColThreads) {
+        const int x = (int)(i % width);
+        const uchar4* at = reinterpret_cast<const uchar4*>(canvas) + i;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        for (int k = max(-R, -x); k <= min(R, width - 1 - x); ++k) {
+            const uchar4 c = at[k];
+            s0 = __dadd_rn(s0, __dmul_rn(g.w[k + R], unit[c.x]));
+            s1 = __dadd_rn(s1, __dmul_rn(g.w[k + R], unit[c.y]));
+            s2 = __dadd_rn(s2, __dmul_rn(g.w[k + R], unit[c.z]));
+        }
+        tmp[i] = s0;
+        tmp[i + n] = s1;
+        tmp[i + 2 * n] = s2;
     }
 }
 
@@ -764,50 +804,58 @@ __device__ __forceinline__ unsigned glow_mix(double cb, double sp, double alpha)
     return (unsigned)max(0, min(255, q));
 }
 
-// the columns' blur of the rows' blur, mixed into the canvas; and the last draw, which needs no neighbours, on top
-template <int R>
+// The columns' blur of the rows' blur, mixed into the canvas; and the last draw, which needs no neighbours, on top.  kOut is
+// one output a thread in a picture of at most kGlowLow rows.
+constexpr int kGlowLow = 3;
+template <int R, int kOut, bool kOneStrip>
 __global__ void __launch_bounds__(kGlowColThreads, 4)
 k_glow_blur_cols_mix(const __grid_constant__ GlowArgs g, unsigned char* __restrict__ canvas, int width, int height,
                      const double* __restrict__ tmp) {
     __shared__ double unit[256];
-    for (int i = threadIdx.x; i < 256; i += kGlowColThreads) unit[i] = __ddiv_rn((double)i, 255.0);
+    const int columns = kOneStrip ? kGlowColThreads : blockDim.x, strips = kOneStrip ? 1 : blockDim.y, strip = kOneStrip ? 0 : threadIdx.y;
+    for (int i = strip * columns + threadIdx.x; i < 256; i += columns * strips) unit[i] = __ddiv_rn((double)i, 255.0);
     __syncthreads();
-    const long long x = (long long)blockIdx.x * kGlowColThreads + threadIdx.x;
+    const long long x = (long long)blockIdx.x * columns + threadIdx.x;
     if (x >= width) return;
     const long long plane = (long long)width * height;
-    for (long long y0 = (long long)blockIdx.y * kGlowColOut; y0 < height; y0 += (long long)gridDim.y * kGlowColOut) {
+    const long long step = (long long)gridDim.y * strips * kOut;
+    for (long long y0 = ((long long)blockIdx.y * strips + strip) * kOut; y0 < height; y0 += step) {
         // input row j of this strip is the picture's row y0 + j - R
-        const int first = y0 < R ? R - (int)y0 : 0, left = (int)min((long long)kGlowColOut + R, height - y0), last = left + R;
+        const int first = y0 < R ? R - (int)y0 : 0, left = (int)min((long long)kOut + R, height - y0), last = left + R;
         unsigned* out = reinterpret_cast<unsigned*>(canvas) + y0 * width + x;
-        unsigned px[kGlowColOut], mixed[kGlowColOut];
+        unsigned px[kOut], mixed[kOut];
 #pragma unroll
-        for (int o = 0; o < kGlowColOut; ++o) {
+        for (int o = 0; o < kOut; ++o) {
             px[o] = o < left ? out[(long long)o * width] : 0u;
             mixed[o] = px[o] & 0xFF000000u;
         }
 #pragma unroll 1
         for (int channel = 0; channel < 3; ++channel) {
             const double* at = tmp + channel * plane + (y0 - R) * width + x;   // read from row j == first on
-            double s[kGlowColOut];
+            double s[kOut];
 #pragma unroll
-            for (int o = 0; o < kGlowColOut; ++o) s[o] = 0.0;
+            for (int o = 0; o < kOut; ++o) s[o] = 0.0;
+            if (kOut == 1) {   // a low picture: few taps are inside it
+                at += (long long)first * width;
+                for (int j = first; j < last; ++j, at += width) s[0] = __dadd_rn(s[0], __dmul_rn(g.w[j], *at));
+            }
 #pragma unroll
-            for (int j = 0; j < kGlowColOut + 2 * R; ++j) {
+            for (int j = 0; kOut > 1 && j < kOut + 2 * R; ++j) {
                 const double v = j >= first && j < last ? *at : 0.0;
                 at += width;
 #pragma unroll
-                for (int o = 0; o < kGlowColOut; ++o)
+                for (int o = 0; o < kOut; ++o)
                     if (j >= o && j <= o + 2 * R) s[o] = __dadd_rn(s[o], __dmul_rn(g.w[j - o], v));
             }
 #pragma unroll
-            for (int o = 0; o < kGlowColOut; ++o) {
+            for (int o = 0; o < kOut; ++o) {
                 unsigned q = glow_mix(unit[(px[o] >> (8 * channel)) & 255u], s[o], g.alpha);
                 if (g.last_alpha != 0.0) q = glow_mix(unit[q], unit[q], g.last_alpha);
                 mixed[o] |= q << (8 * channel);
             }
         }
 #pragma unroll
-        for (int o = 0; o < kGlowColOut; ++o)
+        for (int o = 0; o < kOut; ++o)
             if (o < left) out[(long long)o * width] = mixed[o];
     }
 }
@@ -824,12 +872,25 @@ static cudaError_t launch_glow_blur(double sigma, double alpha, double last_alph
         sum += g.w[k + R];
     }
     for (int k = 0; k <= 2 * R; ++k) g.w[k] /= sum;
-    const dim3 rows((unsigned)(((long long)width + kGlowRowPixels - 1) / kGlowRowPixels), (unsigned)min(height, 65535));
-    k_glow_blur_rows<R><<<rows, kGlowRowThreads, 0, st>>>(g, canvas, width, height, scratch);
+    if (width <= kGlowNarrow) {
+        const long long n = (long long)width * height, blocks = (n + kGlowColThreads - 1) / kGlowColThreads;
+        k_glow_blur_rows_narrow<R><<<(unsigned)min(blocks, 1LL << 20), kGlowColThreads, 0, st>>>(g, canvas, width, n, scratch);
+    } else {
+        const int needed = (width - 1) / kGlowRowOut + 1, lanes = needed <= 16 && height > kGlowTall ? needed : 32;
+        const int across = (int)(((long long)width + lanes * kGlowRowOut - 1) / (lanes * kGlowRowOut)), high = 32 / lanes;
+        const size_t smem = 3 * sizeof(double) * high * (lanes * kGlowRowOut + 2 * R);   // at most 34.6 KB
+        const dim3 grid((unsigned)across, (unsigned)min((height - 1) / high + 1, 65535));
+        auto kern = lanes == 32 ? k_glow_blur_rows<R, true> : k_glow_blur_rows<R, false>;
+        kern<<<grid, kGlowRowThreads, smem, st>>>(g, canvas, width, height, lanes, scratch);
+    }
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
-    const dim3 cols((unsigned)(((long long)width + kGlowColThreads - 1) / kGlowColThreads),
-                    (unsigned)min((height - 1) / kGlowColOut + 1, 65535));
-    k_glow_blur_cols_mix<R><<<cols, kGlowColThreads, 0, st>>>(g, canvas, width, height, scratch);
+    const int out = height <= kGlowLow ? 1 : kGlowColOut;
+    const dim3 block = height > kGlowTall ? column_block(width, kGlowColThreads) : dim3(kGlowColThreads, 1);
+    const long long strips = ((long long)height + out - 1) / out, high = (strips + block.y - 1) / block.y;
+    const dim3 grid((unsigned)((width + block.x - 1LL) / block.x), (unsigned)(high < 65535 ? high : 65535));
+    auto kern = out == 1 ? k_glow_blur_cols_mix<R, 1, true>
+                         : (block.x == kGlowColThreads ? k_glow_blur_cols_mix<R, kGlowColOut, true> : k_glow_blur_cols_mix<R, kGlowColOut, false>);
+    kern<<<grid, block, 0, st>>>(g, canvas, width, height, scratch);
     return cudaGetLastError();
 }
 

@@ -216,9 +216,13 @@ def test_glow_matches_the_cpu_restatement(engine, port):
     assert np.array_equal(engine.glow(tiny), port.glow(tiny))
 
 
-@pytest.mark.parametrize("shape", [(1, 1), (1, 40), (40, 1), (287, 7), (288, 8), (289, 9), (35, 17), (128, 36), (129, 37), (613, 19)])
+@pytest.mark.parametrize("shape", [(1, 1), (1, 40), (40, 1), (287, 7), (288, 8), (289, 9), (35, 17), (128, 36), (129, 37), (613, 19),
+                                   (1, 261), (2, 131), (4, 70), (8, 70), (613, 1), (613, 2), (613, 3), (613, 4), (3, 3), (9, 3), (5, 3),
+                                   (9, 2049), (10, 2079), (18, 2080), (64, 2051), (65, 2050), (72, 2053), (73, 2055), (129, 2049), (144, 2050),
+                                   (145, 2057)])
 def test_glow_at_the_edges_of_its_tiles(engine, port, shape):
-    """Widths around a block's 288 and 128 columns, heights around a strip's 8 rows, pictures smaller than the blur."""
+    """Widths around a block's 288 and 128 columns, heights around a strip's 8 rows, pictures smaller than the blur; narrow
+    and low ones that have kernels of their own, and narrow tall ones, several rows and strips of which make a block."""
     w, h = shape
     rgba = np.random.default_rng(w * 1000 + h).integers(0, 256, size=(h, w, 4), dtype=np.uint8)
     assert np.array_equal(engine.glow(rgba), port.glow(rgba))
@@ -235,18 +239,20 @@ def per_call(engine, call, repeat=10):
     return (time.perf_counter() - t0) / repeat
 
 
-@pytest.mark.parametrize("stage", ["colour"])
+@pytest.mark.parametrize("stage", ["colour", "glow"])
 @pytest.mark.parametrize("width,height", [(8, 131072), (32, 32768), (131072, 8)])
 def test_shape_of_a_picture_does_not_set_its_time(engine, width, height, stage):
     """A million pixels in 8 and 32 columns, and in 8 rows, against 1024 x 1024: blocks that do not fill with such a picture's
     columns took 4 to 15 times as long, full ones take 0.7 to 1.4 times."""
     n = 1 << 20
-    norm, rgba = engine.alloc(8 * n), engine.alloc(4 * n)
+    norm, rgba, scratch = engine.alloc(8 * n), engine.alloc(4 * n), engine.alloc(24 * n)
     norm.from_host(np.random.default_rng(3).uniform(size=n))
-    calls = {"colour": lambda w, h: engine.colorize_device(norm.ptr, w, h, 0, 0, 2, rgba.ptr)}
+    rgba.from_host(np.zeros(4 * n, dtype=np.uint8))
+    calls = {"colour": lambda w, h: engine.colorize_device(norm.ptr, w, h, 0, 0, 2, rgba.ptr),
+             "glow": lambda w, h: L._check(engine.lib.lyap_glow_device(engine.ctx, rgba.ptr, w, h, scratch.ptr))}
     seconds, square = (per_call(engine, lambda: calls[stage](w, h)) for w, h in ((width, height), (1024, 1024)))
     assert seconds < 3.0 * square + 10e-6
-    for b in (norm, rgba):
+    for b in (norm, rgba, scratch):
         b.free()
 
 
