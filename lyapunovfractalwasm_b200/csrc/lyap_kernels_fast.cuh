@@ -112,6 +112,47 @@ struct FastPixel {
     int valid;
 };
 
+// Below kFallen, 1 - 2x and 1 - x round to 1 and r - 2rx to r: a step is x <- r*x and its derivative the parameter itself.
+// A parameter of at most kFallenParam takes such an x to less than 1/2, so that zero is the only way out of (0,1); the
+// comparison is false for NaN, whose derivative is no term of the sum, and for infinity.
+constexpr double kFallen = 0x1p-60, kFallenParam = 0x1p59;
+
+// An orbit that runs down to zero (rA*rB < 1: a whole region of a frame over [0,4]^2 does, each orbit at another step) spends
+// most of its steps below kFallen, where the logarithm of a step's derivative is one of at most three taken beforehand: the
+// same sums, without a table look-up and a polynomial a step.  2048 x 1024 over [0.01,4]^2, "ABAAB" 120 + 1200: fused
+// fp64 4.97 -> 2.32 ms, on the exact orbit 3.60 -> 1.93 (without exits 0.69 and 0.90, as before).
+template <typename T, bool ACC>
+struct Fall {
+    T rA, rB, rC;
+    double zA = 0.0, zB = 0.0, zC = 0.0;   // the parameters' logarithms
+
+    static __device__ __forceinline__ bool applies(T x, T rA, T rB) {   // fp32 orbits are at zero too soon for it to pay
+        return sizeof(T) == 8 && x < (T)kFallen && rA <= (T)kFallenParam && rB <= (T)kFallenParam;
+    }
+    __device__ __forceinline__ Fall(T a, T b, T c) : rA(a), rB(b), rC(c) {
+        if (!ACC) return;
+#pragma unroll 1
+        for (int k = 0; k < 3; ++k) {   // the code of one logarithm
+            const double z = lyap_log_tab((double)(k == 0 ? rC : (k == 1 ? rB : rA)), g_lyap_logtab, 1);
+            zC = zB;
+            zB = zA;
+            zA = z;
+        }
+    }
+    // the first steps of n <= 16 of selector word `word` that are of this kind; their number
+    __device__ __forceinline__ int walk(T& x, double& extra, unsigned word, int n) const {
+        int j = 0;
+        for (; j < n && x > (T)0 && x < (T)kFallen; ++j, word >>= 2) {
+            const unsigned code = word & 3u;
+            if (code >= 2u && !(rC > (T)0 && rC <= (T)kFallenParam)) break;
+            x = FastTraits<T>::mul(code == 0 ? rA : (code == 1 ? rB : rC), x);
+            if (ACC) extra = __dadd_rn(extra, code == 0 ? zA : (code == 1 ? zB : zC));
+        }
+        return j;
+    }
+};
+
+// The reference's rules, one step at a time, for n <= 16 steps of selector word `word`; true when the orbit left (0,1).
 template <typename FL, bool ACC>
 __device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                 typename FL::real rC, unsigned word, int n, unsigned long long* steps) {
@@ -122,8 +163,14 @@ __device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps
     int valid = ps->valid;
     bool dead = false;
     int j = 0;
-    for (; j < n; ++j) {
-        const unsigned sel = (word >> (2 * j)) & 3u;
+    if (Fall<T, ACC>::applies(x, rA, rB)) {
+        j = Fall<T, ACC>(rA, rB, rC).walk(x, extra, word, n);
+        word >>= 2 * (j & 15);   // j == 16: nothing is left
+        dead = !(x > (T)0);
+        if (ACC) valid += j;
+    }
+    for (; j < n && !dead; ++j, word >>= 2) {
+        const unsigned sel = word & 3u;
         const T r = sel == 0 ? rA : (sel == 1 ? rB : rC);
         const T t = F::mul(r, x);
         if (ACC) {
@@ -134,17 +181,36 @@ __device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps
             }
         }
         x = FL::same_orbit ? F::mul(t, F::sub((T)1, x)) : F::fma_(-t, x, t);
-        if (!(x > (T)0 && x < (T)1)) {
-            dead = true;
-            ++j;
-            break;
-        }
+        dead = !(x > (T)0 && x < (T)1);
     }
     *steps += (unsigned long long)j;
     ps->x = x;
     ps->extra = extra;
     ps->valid = valid;
     return dead;
+}
+
+// The steps of a falling orbit from `first` on, of a region whose selector words start at `sel`, up to `end`, to the orbit's own
+// end or to a step that is not of this kind; returns the first step not taken.
+template <typename FL, bool ACC>
+__device__ __noinline__ int fast_fall(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
+                                      typename FL::real rC, const unsigned* sel, int wrap, int first, int end,
+                                      unsigned long long* steps) {
+    using T = typename FL::real;
+    const Fall<T, ACC> fall(rA, rB, rC);
+    T x = ps->x;
+    double extra = ps->extra;
+    int j = first;
+    for (int m = 0, k = 0; k == m && j < end; j += k) {
+        const int in_word = j & (kStepsPerWord - 1);
+        m = min(kStepsPerWord - in_word, end - j);
+        k = fall.walk(x, extra, sel[(j / kStepsPerWord) % wrap] >> (2 * in_word), m);
+    }
+    if (ACC) ps->valid += j - first;
+    *steps += (unsigned long long)(j - first);
+    ps->x = x;
+    ps->extra = extra;
+    return j;
 }
 
 template <typename FL, int P, bool ACC>
@@ -160,55 +226,24 @@ __device__ __forceinline__ void fast_mode_steps(typename FL::real (&x)[P], typen
     }
 }
 
-// Below kFallen, 1 - 2x and 1 - x round to 1 and r - 2rx to r: a step is x <- r*x and its derivative the parameter itself.
-// A parameter of at most kFallenParam takes such an x to less than 1/2, so that zero is the only way out of (0,1); the
-// comparison is false for NaN, whose derivative is no term of the sum, and for infinity.
-constexpr double kFallen = 0x1p-60, kFallenParam = 0x1p59;
-static __device__ __noinline__ double log_of(double d) { return lyap_log_tab(d, g_lyap_logtab, 1); }
-
 // fast_careful_chunk for steps [first, first + n) of a region whose selector words start at `sel`.
-// An orbit that runs down to zero (rA*rB < 1: a whole region of a frame over [0,4]^2 does, each orbit at another step) spends
-// most of them below kFallen, where the logarithm of a step's derivative is one of at most three taken beforehand: the
-// same sums, without a table look-up and a polynomial a step.  2048 x 1024 over [0.01,4]^2, "ABAAB" 120 + 1200: fused
-// fp64 4.97 -> 2.32 ms, on the exact orbit 3.60 -> 1.93 (without exits 0.69 and 0.90, as before).
 template <typename FL, bool ACC>
 __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                 typename FL::real rC, const unsigned* sel, int wrap, int first, int n,
                                                 unsigned long long* steps) {
     using T = typename FL::real;
-    // fp32 orbits are at zero too soon for it to pay
-    const bool may_fall = sizeof(T) == 8 && rA <= (T)kFallenParam && rB <= (T)kFallenParam;
-    bool dead = false, logs = false;
-    double zA = 0.0, zB = 0.0, zC = 0.0;
+    bool dead = false;
     int j = first;
     const int end = first + n;
     while (j < end && !dead) {
+        if (Fall<T, ACC>::applies(ps->x, rA, rB)) {
+            j = fast_fall<FL, ACC>(ps, rA, rB, rC, sel, wrap, j, end, steps);
+            dead = !(ps->x > (T)0);
+            if (dead || j == end) break;
+        }
         const int in_word = j & (kStepsPerWord - 1);
         const int m = min(kStepsPerWord - in_word, end - j);
-        unsigned word = sel[(j / kStepsPerWord) % wrap] >> (2 * in_word);
-        int k = 0;
-        if (may_fall && ps->x < (T)kFallen) {
-            if (ACC && !logs) {
-                zA = log_of((double)rA);
-                zB = log_of((double)rB);
-                zC = log_of((double)rC);
-                logs = true;
-            }
-            T x = ps->x;
-            double extra = ps->extra;
-            for (; k < m && !dead && x < (T)kFallen; ++k, word >>= 2) {
-                const unsigned code = word & 3u;
-                if (code == 2u && !(rC > (T)0 && rC <= (T)kFallenParam)) break;
-                x = FastTraits<T>::mul(code == 0 ? rA : (code == 1 ? rB : rC), x);
-                if (ACC) extra = __dadd_rn(extra, code == 0 ? zA : (code == 1 ? zB : zC));
-                dead = !(x > (T)0);
-            }
-            if (ACC) ps->valid += k;
-            *steps += (unsigned long long)k;
-            ps->x = x;
-            ps->extra = extra;
-        }
-        if (k < m && !dead) dead = fast_careful_chunk<FL, ACC>(ps, rA, rB, rC, word, m - k, steps);
+        dead = fast_careful_chunk<FL, ACC>(ps, rA, rB, rC, sel[(j / kStepsPerWord) % wrap] >> (2 * in_word), m, steps);
         j += m;
     }
     return dead;
@@ -518,8 +553,8 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                         prod[p] = sp[p];
                         FastPixel<T> ps{kSign * sx[p], extra[p], valid[p]};
                         const bool dead =
-                            acc ? fast_careful_steps<FL, true>(&ps, rA[p], rB[p], rC[p], a.sel + word0, wrap, c * kStepsPerWord, n, &my_steps)
-                                : fast_careful_steps<FL, false>(&ps, rA[p], rB[p], rC[p], a.sel + word0, wrap, c * kStepsPerWord, n, &my_steps);
+                            acc ? fast_careful_chunk<FL, true>(&ps, rA[p], rB[p], rC[p], word, n, &my_steps)
+                                : fast_careful_chunk<FL, false>(&ps, rA[p], rB[p], rC[p], word, n, &my_steps);
                         x[p] = kSign * ps.x;
                         extra[p] = ps.extra;
                         valid[p] = ps.valid;
