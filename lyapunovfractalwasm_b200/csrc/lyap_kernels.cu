@@ -349,30 +349,42 @@ __device__ __noinline__ double normalize_any(double val, double t, const lyap_lo
     return __ddiv_rn(1.0, __dadd_rn(1.0, lyap_exp(__dmul_rn(-7.0, __dsub_rn(s, 0.5)))));   // :133
 }
 
+__device__ __forceinline__ double sigmoid_plain(double s) {                             // :133
+    return __drcp_rn(__dadd_rn(1.0, exp_plain(__dmul_rn(-7.0, __dsub_rn(s, 0.5)))));
+}
+
 // Bound by the fp64 pipe and its register reads: 71 fp64 instructions a value in two exponentials and a logarithm.  A value
 // as a frame has them takes the plain functions; sentinels, the minimum itself, NaN and whatever a caller's own min and max
-// make of a value are put right afterwards with the full ones (same bits), so that the common way has no branch in it.
-// 3840 x 2160: 80 us before, 57 now (the pipe alone would take 33); with 4 instead of 8 blocks per SM 60.
+// make of a value are put right afterwards (same bits), so that a thread's common way has no branch in it; a warp that has
+// none but such values leaves it out.
+// 3840 x 2160 with the launch (5 us), a branch a value / no way out for a warp and the load at the top of the loop / as here:
+// ordinary values 85 / 60 / 58 us (the pipe alone 33), half of them sentinels 85 / 65 / 60, all but a few the minimum
+// 48 / 78 / 35; with 4 instead of 8 blocks per SM 3 us more.
 template <int N>
 __device__ __forceinline__ void normalize_some(const double (&val)[N], double (&out)[N], double mn, double range_inv,
                                                const lyap_logtab_entry* tab) {
     double t[N];
-    bool plain[N], all = true;
+    bool plain[N], any = false, all = true;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         t[k] = __dmul_rn(__dsub_rn(val[k], mn), range_inv);                              // :131
         plain[k] = val[k] > -4.0 && t[k] >= 0x1p-300 && t[k] <= 2.0;                      // then val is finite, :130
+        any = any || plain[k];
         all = all && plain[k];
     }
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const double s = pow_plain(plain[k] ? t[k] : 1.0, c_col.y12, tab);               // :132, s < 2.3
-        out[k] = __drcp_rn(__dadd_rn(1.0, exp_plain(__dmul_rn(-7.0, __dsub_rn(s, 0.5)))));   // :133
-    }
-    if (!all) {
+    if (__any_sync(__activemask(), any)) {
 #pragma unroll
         for (int k = 0; k < N; ++k)
-            if (!plain[k]) out[k] = normalize_any(val[k], t[k], tab);
+            out[k] = sigmoid_plain(pow_plain(plain[k] ? t[k] : 1.0, c_col.y12, tab));    // :132, below 2.3
+        if (all) return;
+    }
+    const double least = sigmoid_plain(0.0);                                             // of t = 0
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        if (plain[k]) continue;
+        if (!(val[k] > -4.0 && val[k] <= DBL_MAX)) out[k] = 0.0;                         // :130,135
+        else if (t[k] == 0.0) out[k] = least;
+        else out[k] = normalize_any(val[k], t[k], tab);
     }
 }
 
@@ -383,28 +395,32 @@ k_normalize(const double* __restrict__ v, unsigned long long n, const double* __
     for (int e = threadIdx.x; e < LYAP_LOG_BINS; e += kNormThreads) tab[e] = g_lyap_logtab[e];
     __syncthreads();
     const double mn = minmax[0], mx = minmax[1];
-    const bool degenerate = mn >= mx;                                                    // :122
     const double range_inv = __ddiv_rn(1.0, __dsub_rn(mx, mn));                          // :124-125
     const unsigned long long tid = (unsigned long long)blockIdx.x * kNormThreads + threadIdx.x;
     const unsigned long long nthreads = (unsigned long long)gridDim.x * kNormThreads;
+    if (mn >= mx) {                                                                      // :122
+        for (unsigned long long i = tid; i < n; i += nthreads) out[i] = 0.0;
+        return;
+    }
     const bool aligned = ((reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     if (aligned) {
         const unsigned long long n2 = n / 2;
         const double2* v2 = reinterpret_cast<const double2*>(v);
         double2* o2 = reinterpret_cast<double2*>(out);
+        double2 next = tid < n2 ? v2[tid] : make_double2(0.0, 0.0);   // loaded a round ahead: the branches hold loads back
         for (unsigned long long i = tid; i < n2; i += nthreads) {
-            const double2 q = v2[i];
-            const double val[2] = {q.x, q.y};
-            double r[2] = {0.0, 0.0};
-            if (!degenerate) normalize_some(val, r, mn, range_inv, tab);
+            const double val[2] = {next.x, next.y};
+            if (i + nthreads < n2) next = v2[i + nthreads];
+            double r[2];
+            normalize_some(val, r, mn, range_inv, tab);
             o2[i] = make_double2(r[0], r[1]);
         }
     }
     // values of a misaligned array, the last of an odd number
     for (unsigned long long i = aligned ? (n & ~1ull) + tid : tid; i < n; i += nthreads) {
         const double val[1] = {v[i]};
-        double r[1] = {0.0};
-        if (!degenerate) normalize_some(val, r, mn, range_inv, tab);
+        double r[1];
+        normalize_some(val, r, mn, range_inv, tab);
         out[i] = r[0];
     }
 }

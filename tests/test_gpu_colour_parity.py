@@ -1,6 +1,8 @@
 """GPU parity of the colour stage on the large benchmark frames: normalizeData's whole-frame min/max
 (reference src/lyapunov_fractal.hpp:110-125), its map (:127-137) and the page's 3x3 mean + palette + byte store
 (web/fractal_renderer.js:283-311,207-281,191-198), against the CPU oracle.  Bar: identical fp64 words and bytes."""
+import time
+
 import numpy as np
 import pytest
 
@@ -140,6 +142,30 @@ def test_normalise_edges_and_special_values(engine, port, n):
             at = rng.integers(0, n, size=max(1, n // 5))
             values[at] = rng.choice([-5.0, -4.0, -3.9999999, np.nan, np.inf, -np.inf, 0.0, 1e-310, -3.0, 1.2], size=at.size)
         assert same_bits(engine.normalize_data(values), port.normalize(values)), special
+
+
+def test_normalise_of_a_flat_frame_takes_no_longer(engine, port):
+    """Eight million values, all but the last 20 the minimum, against as many ordinary ones: 1.3 times the time when a warp of
+    them went the common way and then put each right, 0.6 so.  Same bits as the oracle at the seam."""
+    n = 1 << 23
+    d_v, d_out, d_mm = engine.alloc(8 * n), engine.alloc(8 * n), engine.alloc(16)
+    flat = np.full(n, 0.25)
+    flat[-20:] = np.linspace(0.3, 0.5, 20)
+    best = {}
+    for name, values in (("ordinary", np.random.default_rng(1).uniform(-3.0, 1.2, n)), ("flat", flat)):
+        d_v.from_host(values)
+        engine.minmax_device(d_v.ptr, n, d_mm.ptr)
+        for _ in range(5):
+            engine.sync()
+            t0 = time.perf_counter()
+            for _ in range(10):
+                engine.normalize_device(d_v.ptr, n, d_mm.ptr, d_out.ptr)
+            engine.sync()
+            best[name] = min(best.get(name, 1.0), time.perf_counter() - t0)
+    assert same_bits(d_out.to_host(np.float64, 100, 8 * (n - 100)), port.normalize(flat)[-100:])
+    assert best["flat"] < best["ordinary"]
+    for b in (d_v, d_out, d_mm):
+        b.free()
 
 
 @pytest.mark.parametrize("n", [2, 3, 4, 5, 64, 4097, 700001])
