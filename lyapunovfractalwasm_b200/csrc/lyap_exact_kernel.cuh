@@ -136,9 +136,12 @@ __device__ __forceinline__ double log_fast(double d, unsigned lane_off) {
     return __dadd_rn(hi, s);
 }
 
-// careful_chunk for steps [first, first + n) of a region whose selector words start at `sel` (n <= 64).
+// Most steps between two exit tests; what careful_steps may be called with.
+constexpr int kMaxChunk = 64;
+
+// careful_chunk for steps [first, first + n) of a region whose selector words start at `sel` (n <= kMaxChunk).
 // An orbit that has fallen below 2^-600 and whose parameters (positive: the others are sentinels) are at most 256 stays
-// below 2^-88 for these steps, where 1 - 2x and 1 - x round to 1: the derivative is the parameter itself, with one of at
+// below 2^-88 for these steps (2^(8 kMaxChunk - 600)), where 1 - 2x and 1 - x round to 1: the derivative is the parameter itself, with one of at
 // most three logarithms, and a step is a multiplication, an addition and the exit test.  That is how nearly every orbit of
 // a frame over [0,4]^2 that ends does end (x runs down to zero where rA*rB < 1), a whole region's after one another.
 // Measured, 800 x 800 over [0.01,3.99]^2, "AB" 100 + 1000: 0.745 -> 0.702 ms (0.645 for a window without exits).
@@ -370,6 +373,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
             // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code)
             constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = 2, CS = CB * BS * REP;
+            static_assert(CS <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
             const unsigned* sel = a.sel + word0;
             int s = 0;
             while (s < nsteps) {
@@ -434,6 +438,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             continue;
         }
         // generic walk: the selector words one after the other, exit tests after every second full word
+        static_assert(2 * kStepsPerWord <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
         const unsigned* sel = a.sel + word0;
         int s = 0, wi = 0;
         while (s < nsteps) {
