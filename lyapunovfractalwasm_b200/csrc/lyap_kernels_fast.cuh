@@ -1,8 +1,8 @@
 // lyap_kernels_fast.cuh -- fast-mode lambda kernels (included by lyap_kernels.cu after lyap_exact_kernel.cuh, and, as
 // text, by the run-time specialiser).
 //
-// Same pixel mapping, sequence handling, sentinel and early-exit rules as the exact kernel, but the
-// arithmetic is rearranged for speed and is NOT bit-compatible with the reference:
+// Same sequence handling, sentinel and early-exit rules as the exact kernel; a thread owns P neighbouring pixels of a
+// row.  The arithmetic is rearranged for speed and is NOT bit-compatible with the reference:
 //   t = r*x;  deriv = fma(-2,t,r) = r(1-2x);  x' = fma(-t,x,t) = r x (1-x)         (4 fused ops/step)
 // and instead of one log per step the |deriv| are multiplied together; the product's exponent is
 // moved into an integer at least every 32 (fp64) or 20 (fp32) steps, and one log of the remaining mantissa is
@@ -120,7 +120,7 @@ constexpr double kFallen = 0x1p-60, kFallenParam = 0x1p59;
 // An orbit that runs down to zero (rA*rB < 1: a whole region of a frame over [0,4]^2 does, each orbit at another step) spends
 // most of its steps below kFallen, where the logarithm of a step's derivative is one of at most three taken beforehand: the
 // same sums, without a table look-up and a polynomial a step.  2048 x 1024 over [0.01,4]^2, "ABAAB" 120 + 1200: fused
-// fp64 4.97 -> 2.32 ms, on the exact orbit 3.60 -> 1.93 (without exits 0.69 and 0.90, as before).
+// fp64 5.11 -> 2.07 ms, on the exact orbit 3.74 -> 1.82 (over [2.5,4]^2, without exits, 0.67 and 0.88, as before).
 template <typename T, bool ACC>
 struct Fall {
     T rA, rB, rC;
@@ -154,8 +154,8 @@ struct Fall {
 
 // The reference's rules, one step at a time, for n <= 16 steps of selector word `word`; true when the orbit left (0,1).
 template <typename FL, bool ACC>
-__device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
-                                                typename FL::real rC, unsigned word, int n, unsigned long long* steps) {
+__device__ __forceinline__ bool fast_careful_body(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
+                                                  typename FL::real rC, unsigned word, int n, unsigned long long* steps) {
     using T = typename FL::real;
     using F = FastTraits<T>;
     T x = ps->x;
@@ -190,12 +190,20 @@ __device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps
     return dead;
 }
 
+// The same as a function of its own, for the generic walk.  Neither it nor fast_careful_steps calls another: a second level of
+// calls shows in the registers that the kernels' own loops have left.
+template <typename FL, bool ACC>
+__device__ __noinline__ bool fast_careful_chunk(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
+                                                typename FL::real rC, unsigned word, int n, unsigned long long* steps) {
+    return fast_careful_body<FL, ACC>(ps, rA, rB, rC, word, n, steps);
+}
+
 // The steps of a falling orbit from `first` on, of a region whose selector words start at `sel`, up to `end`, to the orbit's own
 // end or to a step that is not of this kind; returns the first step not taken.
 template <typename FL, bool ACC>
-__device__ __noinline__ int fast_fall(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
-                                      typename FL::real rC, const unsigned* sel, int wrap, int first, int end,
-                                      unsigned long long* steps) {
+__device__ __forceinline__ int fast_fall(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
+                                         typename FL::real rC, const unsigned* sel, int wrap, int first, int end,
+                                         unsigned long long* steps) {
     using T = typename FL::real;
     const Fall<T, ACC> fall(rA, rB, rC);
     T x = ps->x;
@@ -226,7 +234,7 @@ __device__ __forceinline__ void fast_mode_steps(typename FL::real (&x)[P], typen
     }
 }
 
-// fast_careful_chunk for steps [first, first + n) of a region whose selector words start at `sel`.
+// fast_careful_body for steps [first, first + n) of a region whose selector words start at `sel` (specialised walk).
 template <typename FL, bool ACC>
 __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                 typename FL::real rC, const unsigned* sel, int wrap, int first, int n,
@@ -243,7 +251,7 @@ __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps
         }
         const int in_word = j & (kStepsPerWord - 1);
         const int m = min(kStepsPerWord - in_word, end - j);
-        dead = fast_careful_chunk<FL, ACC>(ps, rA, rB, rC, sel[(j / kStepsPerWord) % wrap] >> (2 * in_word), m, steps);
+        dead = fast_careful_body<FL, ACC>(ps, rA, rB, rC, sel[(j / kStepsPerWord) % wrap] >> (2 * in_word), m, steps);
         j += m;
     }
     return dead;
