@@ -623,13 +623,15 @@ __device__ __forceinline__ unsigned colorize_inner(const double (&above)[3], con
 
 // A thread takes one column of kColorRows rows: its rows' values and their left and right neighbours are loaded once, side by
 // side across the warp, and stay in registers for the pixels above and below.  A block is up to 256 columns wide and, in a
-// narrow frame, as many strips high as fill it.  A warp with a pixel at the frame's edge loads -0 for a neighbour that is
-// not there, which leaves any sum as it is.  The palette is a template parameter: its code is then straight-line.
-// 3840 x 2160, aurora / solarflare (the cheapest palette): 95 / 85 us with nine loads behind tests a pixel, 66 / 55 us with
-// four pixels of a row to a thread (18 loads, but 32 bytes apart across the warp), 52 / 38 us as here; with the tests for
-// the rows that exist inside every strip's code, 64-bit and uniform, it was 82 / 68.
+// narrow frame, as many strips high as fill it.  A warp with a pixel at the frame's edge goes row by row and
+// takes -0 for a neighbour that is not there, which leaves any sum as it is.  The palette is a template parameter: its code is
+// then straight-line.
+// 3840 x 2160 with the launch, aurora / solarflare (the cheapest palette): 102 / 90 us with nine loads behind tests a pixel,
+// 51 / 41 us as here.  Four pixels of a row to a thread (18 loads, but 32 bytes apart across the warp) cost 14 / 17 us more,
+// tests for the rows that exist inside every strip's code 30, the edge's code unrolled like the strip's 4 / 5 (spills; as many
+// with 3 blocks an SM).
 // Solarflare, two million pixels in 32 / 8 columns: 31 / 32 us with nine loads a pixel, 117 / 432 in blocks of 256 columns of
-// one strip, 19 / 21 so.
+// one strip, 20 / 21 so.
 constexpr int kColorRows = 4;
 
 template <int PALETTE>
@@ -648,8 +650,8 @@ k_colorize(const double* __restrict__ norm, int width, long long rows, int rows_
         const double* at = norm + (y0 - 1) * width + x;   // in the row above: read only if that exists
         const bool whole = (y0 > 0 || rows_above) && (y0 + kColorRows < rows || (y0 + kColorRows == rows && rows_below));
         unsigned int* out = rgba + y0 * width + x;
-        double v[kColorRows + 2][3];
         if (__all_sync(__activemask(), whole && x > 0 && x < width - 1)) {
+            double v[kColorRows + 2][3];
 #pragma unroll
             for (int r = 0; r < kColorRows + 2; ++r) {
 #pragma unroll
@@ -663,23 +665,29 @@ k_colorize(const double* __restrict__ norm, int width, long long rows, int rows_
             }
         } else {
             const bool left = x > 0, right = x < width - 1;
-            const int there = (int)min(rows - y0, (long long)kColorRows + 1);             // own rows of the strip and below it
-            const int first = y0 > 0 || rows_above ? 0 : 1, last = there + (there <= kColorRows && rows_below ? 1 : 0);
-#pragma unroll
-            for (int r = 0; r < kColorRows + 2; ++r) {
+            const int columns = 1 + left + right, there = (int)min(rows - y0, (long long)kColorRows);
+            const int first = y0 > 0 || rows_above ? 0 : 1, last = y0 + there < rows || rows_below ? there + 1 : there;
+            double w[3][3];   // the rows above, at and below the pixel
+            const auto load = [&](int r, double (&q)[3]) {
                 const bool row = r >= first && r <= last;
-                v[r][0] = row && left ? at[-1] : -0.0;
-                v[r][1] = row ? at[0] : -0.0;
-                v[r][2] = row && right ? at[1] : -0.0;
+                q[0] = row && left ? at[-1] : -0.0;
+                q[1] = row ? at[0] : -0.0;
+                q[2] = row && right ? at[1] : -0.0;
                 at += width;
-            }
-            const int columns = 1 + left + right;
-#pragma unroll
-            for (int r = 0; r < kColorRows; ++r) {
-                if (r >= there) break;
+            };
+            load(0, w[0]);
+            load(1, w[1]);
+#pragma unroll 1
+            for (int r = 0; r < there; ++r) {
+                load(r + 2, w[2]);
                 const int count = columns * (1 + (r >= first) + (r + 2 <= last));
-                *out = colorize_inner<PALETTE>(v[r], v[r + 1], v[r + 2], (double)count, c_col.recip[count], tab);
+                *out = colorize_inner<PALETTE>(w[0], w[1], w[2], (double)count, c_col.recip[count], tab);
                 out += width;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    w[0][k] = w[1][k];
+                    w[1][k] = w[2][k];
+                }
             }
         }
     }
