@@ -188,31 +188,17 @@ def test_default_mode_compiles_in_the_background(engine, port):
 
 
 @pytest.mark.parametrize("iterations", [1, 15, 16, 17, 20, 21, 161, 333])
-def test_packed_fp32_step_is_the_one_wide_step(engine, kernel_path, iterations):
-    """The two-wide fp32 step over both walks (specialised and generic) against the one-wide step restated here: two
-    accumulated products of float32 fma's, taken in float64, where a product of two float32 is exact and the sum of it and
-    a float32 is rounded once more -- a value that falls on a tie then differs by an ulp of float32, 6e-8, which a stable
-    orbit does not amplify: 3e-7 bounds a derivative's difference."""
-    kw = dict(min_x=2.2, max_x=2.9, min_y=2.3, max_y=2.95, width=35, height=9, sequence="AAB", iterations=iterations, warmup=40)
-    x = np.full((9, 35), 0.5, dtype=np.float32)
-    dx, dy = (kw["max_x"] - kw["min_x"]) / 34.0, (kw["max_y"] - kw["min_y"]) / 8.0
-    ra = np.broadcast_to((kw["min_x"] + dx * np.arange(35)).astype(np.float32), x.shape)
-    rb = np.broadcast_to((kw["min_y"] + dy * np.arange(9)).astype(np.float32)[:, None], x.shape)
-    total, smallest = np.zeros(x.shape), 1.0
-    for i in range(40 + iterations):
-        r = (ra if "AAB"[i % 3] == "A" else rb).astype(np.float32)
-        tt = r * x
-        if i >= 40:
-            deriv = np.abs((r.astype(np.float64) - 2.0 * tt).astype(np.float32)).astype(np.float64)
-            total, smallest = total + np.log(deriv), min(smallest, deriv.min())
-        x = (tt.astype(np.float64) - tt.astype(np.float64) * x).astype(np.float32)
-    want = total / (iterations * np.log(2.0))
-    got = {}
+def test_packed_fp32_step_is_the_one_wide_step(engine, port, kernel_path, iterations):
+    """The two-wide fp32 step over both walks (specialised and generic) against the one-wide step restated in C++ floats: the
+    same exits at the same steps, chaotic pixels included, and lambdas that differ by the running product's roundings, at
+    most 2^-24 of a factor a step: 2^-24 / ln 2 of the mean (and its square, and the double's)."""
+    kw = dict(min_x=2.2, max_x=4.05, min_y=2.3, max_y=4.02, width=35, height=9, sequence="AAB", iterations=iterations, warmup=40)
+    want, steps = port.fused_lambda(**kw, single=True)
     for path in ("jit", "generic"):
         kernel_path(path)
-        got[path] = engine.compute_fractal(L.make_params(**kw, mode=L.MODE_FAST_FP32))
-        assert np.max(np.abs(got[path] - want)) < 3e-7 / smallest / np.log(2.0) + 1e-6, path   # + the products' roundings
-    assert np.max(np.abs(got["jit"] - got["generic"])) < 2e-6
+        r = engine.render(L.make_params(**kw, mode=L.MODE_FAST_FP32), want=("lambda",))
+        assert r["stats"].executed_steps == steps, path
+        assert np.max(np.abs(r["lambda"] - want)) < 1.001 * 2.0 ** -24 / np.log(2.0), path
 
 
 @pytest.mark.parametrize("kw", [
