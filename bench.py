@@ -49,12 +49,12 @@ CFG4 = dict(min_x=2.0, max_x=4.0, min_y=2.0, max_y=4.0, width=65536, height=6553
             iterations=1000, warmup=100)
 # fp64 instructions per logistic step in the exact kernel's main path, counted from its source:
 #   warm-up step      3  (r*x, 1-x, product)
-#   accumulated step 13  (fma(-2,x,1), r*|.|, 7 for the log incl. its last addition, sum +=, r*x, 1-x, product)
+#   accumulated step 13  (0.5-x, r*|.|, 7 for the log incl. its last addition, sum +=, r*x, 1-x, product)
 # The log's other two products, e*ln2hi and (e-1023)*ln2lo, come from a 4096-entry shared-memory table.
 OPS_WARM, OPS_ACC = 3, 13
-# the same steps in flops (a fused multiply-add counts 2): warm-up 3 (none fused); accumulated 19 = 13 instructions,
-# 6 of them fused (fma(-2,x,1), r = fma(d,inv,-1), three for the cubic, s = fma(r,w,klo))
-FLOPS_WARM, FLOPS_ACC = 3, 19
+# the same steps in flops (a fused multiply-add counts 2): warm-up 3 (none fused); accumulated 18 = 13 instructions,
+# 5 of them fused (r = fma(d,inv,-1), three for the cubic, s = fma(r,w,klo))
+FLOPS_WARM, FLOPS_ACC = 3, 18
 FAST_OPS = 4   # fast modes: 4 instructions per step on the fp64 / fp32 pipe, 2 of them fused (6 flops)
 FAST_FLOPS = 6
 
@@ -585,8 +585,8 @@ def main():
             "achieved": pipe["achieved"], "peak": pipe["peak"], "unit": "T thread-instr/s", "frac": pipe["frac"],
             "frac_flops": pipe["frac_flops"], "achieved_tflops": pipe["achieved_tflops"], "peak_tflops": pipe["peak_tflops"],
             "flops_note": "a fused multiply-add counts 2 flops, so the flop peak is 2 x the issue-rate peak; the exact mode may fuse "
-                          "only where the reference's rounding allows (6 of its 13 instructions per accumulated step), which "
-                          "caps frac_flops at 19/26 of frac",
+                          "only where the reference's rounding allows (5 of its 13 instructions per accumulated step), which "
+                          "caps frac_flops at 18/26 of frac",
             "peak_source": "measured in this run: independent FMA chains on all SMs (lyap_fp64_peak / lyap_fp32_peak); "
                            "MEASURED_PEAKS.json has no fp64/fp32 vector entry",
             "instr_per_step": {"warmup": OPS_WARM, "accumulated": OPS_ACC} if mode == L.MODE_EXACT else FAST_OPS,

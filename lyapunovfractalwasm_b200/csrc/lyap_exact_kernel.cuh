@@ -14,8 +14,8 @@ static __device__ const lyap_logtab_entry g_lyap_logtab[LYAP_LOG_BINS] = {LYAP_L
 // ---------------------------------------------------------------------------------------------
 // Exact lambda kernel.
 //
-// One thread owns P horizontally adjacent pixels for their whole orbit: x, the running log sum and
-// the two parameter values stay in registers.  The per-step A/B(/C) choice is the same for every
+// One thread owns P pixels of one column, one below another, for their whole orbit: x, the running log sum
+// and the parameter values stay in registers.  The per-step A/B(/C) choice is the same for every
 // pixel, so steps are taken in groups of U whose pattern (e.g. "AB", "BA") picks, by one warp-uniform
 // multiway branch, a straight-line body compiled for exactly that pattern: no per-step select or branch.
 // Inside a body the orbit runs ahead and the U*P logarithms that hang off it are independent chains.
@@ -25,7 +25,7 @@ static __device__ const lyap_logtab_entry g_lyap_logtab[LYAP_LOG_BINS] = {LYAP_L
 // quarter warp, whose 8 lanes then hit 8 different 16-byte bank groups whatever their indices are,
 // so the lookups never conflict.
 //
-// Steps run in chunks of 16 to about 40 without per-step exit tests.  That is sound because leaving (0,1)
+// Steps run in chunks of 32 to kMaxChunk (fewer at a region's end) without per-step exit tests.  That is sound because leaving (0,1)
 // is permanent for x <- r x (1-x) with r > 0 (x >= 1 gives x <= 0 next, x <= 0 stays <= 0, NaN stays
 // NaN), so testing x after the chunk finds every exit, and the only other irregular event, a zero
 // derivative (x == 0.5 exactly, skipped and not counted by the reference, :71-74), has exponent field 0,
@@ -141,9 +141,10 @@ constexpr int kMaxChunk = 64;
 
 // careful_chunk for steps [first, first + n) of a region whose selector words start at `sel` (n <= kMaxChunk).
 // An orbit that has fallen below 2^-600 and whose parameters (positive: the others are sentinels) are at most 256 stays
-// below 2^-88 for these steps (2^(8 kMaxChunk - 600)), where 1 - 2x and 1 - x round to 1: the derivative is the parameter itself, with one of at
-// most three logarithms, and a step is a multiplication, an addition and the exit test.  That is how nearly every orbit of
-// a frame over [0,4]^2 that ends does end (x runs down to zero where rA*rB < 1), a whole region's after one another.
+// below 2^-88 (2^(8 kMaxChunk - 600)) for these steps, where 1 - 2x and 1 - x round to 1: the derivative is the parameter
+// itself, with one of at most three logarithms, and a step is a multiplication, an addition and the exit test.  That is how
+// nearly every orbit of a frame over [0,4]^2 that ends does end (x runs down to zero where rA*rB < 1), a whole region's after
+// one another.
 // Measured, 800 x 800 over [0.01,3.99]^2, "AB" 100 + 1000: 0.745 -> 0.702 ms (0.645 for a window without exits).
 template <bool ACC>
 __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB, double rC, const unsigned* sel, int wrap, int first,
