@@ -407,7 +407,7 @@ k_normalize(const double* __restrict__ v, unsigned long long n, const double* __
         const unsigned long long n2 = n / 2;
         const double2* v2 = reinterpret_cast<const double2*>(v);
         double2* o2 = reinterpret_cast<double2*>(out);
-        double2 next = tid < n2 ? v2[tid] : make_double2(0.0, 0.0);   // loaded a round ahead: the branches hold loads back
+        double2 next = tid < n2 ? v2[tid] : make_double2(0.0, 0.0);   // loaded a turn of the loop ahead: the branches hold loads back
         for (unsigned long long i = tid; i < n2; i += nthreads) {
             const double val[2] = {next.x, next.y};
             if (i + nthreads < n2) next = v2[i + nthreads];
