@@ -87,7 +87,7 @@ typedef struct lyap_ctx lyap_ctx;      /* one device, one stream, scratch buffer
 typedef void (*lyap_progress_fn)(double fraction);
 
 typedef struct lyap_render_stats {
-    uint64_t executed_steps;           /* logistic updates actually performed (early exits excluded) */
+    uint64_t executed_steps;           /* logistic updates of the orbits up to their exits, as the reference performs them */
     uint64_t nominal_steps;            /* pixels * (warmup + iterations) */
     double lambda_min, lambda_max;     /* over finite values > -4 (normalizeData's filter) */
     float ms_lambda, ms_minmax, ms_normalize, ms_colorize, ms_total_device, ms_copies;
@@ -123,7 +123,9 @@ int lyap_copy_to_device(lyap_ctx* ctx, void* dev, const void* host, size_t bytes
 
 /* FractalComputer::computeFractal (src/lyapunov_fractal.hpp:27-102) for rows [row_begin,row_end).
  * d_lambda: rows*width doubles, or NULL; d_lambda32: same count of floats ((float)lambda), or NULL.
- * d_steps: one uint64 the kernel ADDS executed steps to, or NULL. */
+ * d_steps: one uint64 the kernel ADDS executed steps to, or NULL.  An orbit that has come back to an earlier value is
+ * not walked any further -- the rest of its sum is added up from one turn of its cycle, to the same bits -- but its
+ * steps count all the same: they are the reference's.  lyap_cycle_steps says how many were not walked. */
 int lyap_lambda_device(lyap_ctx* ctx, const lyap_params* p, double* d_lambda, float* d_lambda32,
                        uint64_t* d_steps);
 
@@ -293,6 +295,10 @@ int lyap_selector_code(const lyap_params* params, int region, int64_t step, int*
 int lyap_group_patterns(const lyap_params* params, int* groups, uint64_t* warmup_patterns, uint64_t* accumulation_patterns);
 
 /* ---- measurement ---- */
+
+/* *steps = how many of the executed steps of this context's lambda launches so far were taken from an orbit's cycle
+ * instead of being walked (see lyap_lambda_device); waits for the context's stream. */
+int lyap_cycle_steps(lyap_ctx* ctx, uint64_t* steps);
 
 /* Issue-rate micro-benchmark of the fp64 pipe on the context's device: independent DFMA chains,
  * all SMs.  Writes thread-level fp64 instructions per second. */

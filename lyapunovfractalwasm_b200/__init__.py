@@ -119,6 +119,7 @@ ABI = {
                                           ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(_P), ctypes.POINTER(_P),
                                           ctypes.POINTER(RenderStats)]),
     "lyap_minmax_device_noalloc": (ctypes.c_int, [_P, ctypes.c_uint64, _P, _P]),
+    "lyap_cycle_steps": (ctypes.c_int, [_P, c_u64_p]),
     "lyap_fp64_peak": (ctypes.c_int, [_P, c_double_p]),
     "lyap_fp32_peak": (ctypes.c_int, [_P, c_double_p]),
 }
@@ -423,6 +424,12 @@ class Engine:
 
     def sync(self):
         _check(self.lib.lyap_sync(self.ctx))
+
+    def cycle_steps(self):
+        """Steps of this engine's lambda launches so far that were taken from an orbit's cycle instead of being walked."""
+        v = ctypes.c_uint64(0)
+        _check(self.lib.lyap_cycle_steps(self.ctx, ctypes.byref(v)))
+        return v.value
 
     def fp64_peak(self):
         v = ctypes.c_double()

@@ -57,7 +57,7 @@ struct lyap_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
     Buffer lambda, lambda32, norm, rgba;   // frame-sized work buffers of the host-pointer entry points
-    void* small = nullptr;                 // [0,16) min/max, [16,24) step counter, then min/max scratch
+    void* small = nullptr;                 // [0,16) min/max, [16,24) step counter, [24,32) steps taken from cycles, [32,40) tile queue, then min/max scratch
     cudaEvent_t ev[8] = {};
     std::vector<cudaEvent_t> chunk_events;
 };
@@ -68,7 +68,23 @@ double* ctx_minmax(lyap_ctx* c) { return static_cast<double*>(c->small); }
 unsigned long long* ctx_steps(lyap_ctx* c) {
     return reinterpret_cast<unsigned long long*>(static_cast<char*>(c->small) + 16);
 }
-void* ctx_scratch(lyap_ctx* c) { return static_cast<char*>(c->small) + 32; }
+unsigned long long* ctx_cycle_steps(lyap_ctx* c) { return ctx_steps(c) + 1; }
+unsigned* ctx_queue(lyap_ctx* c) { return reinterpret_cast<unsigned*>(static_cast<char*>(c->small) + 32); }
+constexpr size_t kSmallHead = 64;
+void* ctx_scratch(lyap_ctx* c) { return static_cast<char*>(c->small) + kSmallHead; }
+
+// The context's tile queue, or null for a launch that another of the same context might overlap: launches of a context follow
+// one another on its stream, but a captured one runs wherever and whenever its graph does, and cudaStreamPerThread stands for
+// several streams.
+unsigned* queue_for_launch(lyap_ctx* c) {
+    if (c->stream == cudaStreamPerThread) return nullptr;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return status == cudaStreamCaptureStatusNone ? ctx_queue(c) : nullptr;
+}
 
 int ensure(lyap_ctx* c, Buffer& b, size_t bytes) {
     if (b.cap >= bytes) return LYAP_OK;
@@ -153,6 +169,25 @@ int build_args(const lyap_params* p, lyap::LambdaArgs* a, Geometry* g) {
     for (long long i = 0; i < wu_stored; ++i) a->sel[i / 16] |= code(i) << (2 * (i % 16));
     for (long long i = 0; i < acc_stored; ++i)
         a->sel[wu_words + i / 16] |= code((long long)p->warmup + i) << (2 * (i % 16));
+    // the shortest period of the accumulation's selectors (in a wrapped region one that goes into the sequence's), and the generic
+    // kernel's chunk: whole periods, as many as hold the cycles that there are (of one, two, four, ... periods first, then of three)
+    const auto acc_code = [&](long long i) { return (a->sel[wu_words + i / 16] >> (2 * (i % 16))) & 3u; };
+    const auto repeats = [&](int t) {
+        if (acc_words < acc_need && seq_len % t != 0) return false;
+        for (long long i = t; i < acc_stored; ++i)
+            if (acc_code(i) != acc_code(i - t)) return false;
+        return true;
+    };
+    int period = 1;
+    while (period <= lyap::kMaxChunk && !repeats(period)) ++period;
+    a->acc_chunk = 2 * lyap::kStepsPerWord;
+    if (period <= lyap::kMaxChunk) {
+        a->acc_period = period;
+        for (int periods : {48, 24, 12, 8, 4, 2, 1}) {
+            a->acc_chunk = periods * period;
+            if (a->acc_chunk <= (periods == 2 ? lyap::kMaxChunk : 64)) break;
+        }
+    }
     const double c = p->c_value;
     a->fast_ok_c = (!seq_has_c || (c > 0x1p-20 && c < 0x1p20)) ? 1 : 0;
     g->row_begin = rb;
@@ -161,8 +196,10 @@ int build_args(const lyap_params* p, lyap::LambdaArgs* a, Geometry* g) {
     return LYAP_OK;
 }
 
-int launch_lambda(lyap_ctx* c, int mode, const lyap::LambdaArgs& a, double* d64, float* d32, unsigned long long* steps) {
+int launch_lambda(lyap_ctx* c, int mode, lyap::LambdaArgs& a, double* d64, float* d32, unsigned long long* steps) {
     Range range("lyap: lambda");
+    a.cycle_steps = ctx_cycle_steps(c);
+    a.queue = queue_for_launch(c);
     cudaError_t e;
     if (mode == LYAP_MODE_EXACT) e = lyap::launch_lambda_exact(a, d64, d32, steps, c->sm_count, c->stream);
     else if (mode == LYAP_MODE_FAST_FP64) e = lyap::launch_lambda_fast64(a, d64, d32, steps, c->sm_count, c->stream);
@@ -293,8 +330,8 @@ int lyap_create(lyap_ctx** out, int device) {
     c->device = device;
     c->sm_count = prop.multiProcessorCount;
     cudaError_t e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&c->small, 32 + lyap::kMinmaxScratchBytes);
-    if (e == cudaSuccess) e = cudaMemset(c->small, 0, 32 + lyap::kMinmaxScratchBytes);
+    if (e == cudaSuccess) e = cudaMalloc(&c->small, kSmallHead + lyap::kMinmaxScratchBytes);
+    if (e == cudaSuccess) e = cudaMemset(c->small, 0, kSmallHead + lyap::kMinmaxScratchBytes);
     for (int i = 0; i < 8 && e == cudaSuccess; ++i) e = cudaEventCreate(&c->ev[i]);
     if (e != cudaSuccess) {
         lyap_destroy(c);
@@ -641,6 +678,11 @@ static int peak_common(lyap_ctx* c, bool fp64, double* out) {
     }
     *out = best;
     return LYAP_OK;
+}
+
+int lyap_cycle_steps(lyap_ctx* c, uint64_t* steps) {
+    if (!steps) return fail(LYAP_ERR_INVALID, "null pointer");
+    return lyap_copy_to_host(c, steps, c ? ctx_cycle_steps(c) : nullptr, sizeof(*steps));
 }
 
 int lyap_fp64_peak(lyap_ctx* c, double* instr_per_second) { return peak_common(c, true, instr_per_second); }

@@ -9,6 +9,8 @@ namespace lyap {
 // its share of the table stores one period of the sequence in whole words (lcm(len, 16) steps) and repeats
 // it: word w of a region is sel[word0 + w % wrap].
 constexpr int kStepsPerWord = 16;
+// Most steps between two exit tests of the exact kernels.
+constexpr int kMaxChunk = 80;
 constexpr int kMaxSelWords = 896;  // 14336 distinct steps through kernel parameters (kernel parameter space is 4 KB)
 
 struct LambdaArgs {
@@ -21,6 +23,10 @@ struct LambdaArgs {
     int acc_word0;
     int fast_ok_c;         // c_value is positive, finite and of ordinary magnitude (or unused)
     int wu_wrap, acc_wrap; // words after which each region's selectors repeat (>= the region's words when it is stored whole)
+    int acc_period;        // steps after which the accumulation's selectors repeat, 0 when that is more than kMaxChunk
+    int acc_chunk;         // steps between two exit tests of the generic exact kernel: a multiple of acc_period, if there is one
+    unsigned* queue;       // exact kernel: tiles handed out so far and warps that are done, both zero between launches; null: no queue
+    unsigned long long* cycle_steps;   // counts steps taken from an orbit's cycle instead of being walked (may be null)
     unsigned int sel[kMaxSelWords];
 };
 

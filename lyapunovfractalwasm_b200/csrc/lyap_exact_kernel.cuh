@@ -136,12 +136,9 @@ __device__ __forceinline__ double log_fast(double d, unsigned lane_off) {
     return __dadd_rn(hi, s);
 }
 
-// Most steps between two exit tests; what careful_steps may be called with.
-constexpr int kMaxChunk = 64;
-
 // careful_chunk for steps [first, first + n) of a region whose selector words start at `sel` (n <= kMaxChunk).
-// An orbit that has fallen below 2^-600 and whose parameters (positive: the others are sentinels) are at most 256 stays
-// below 2^-88 (2^(8 kMaxChunk - 600)) for these steps, where 1 - 2x and 1 - x round to 1: the derivative is the parameter
+// An orbit that has fallen below 2^-740 and whose parameters (positive: the others are sentinels) are at most 256 stays
+// below 2^-100 (2^(8 kMaxChunk - 740)) for these steps, where 1 - 2x and 1 - x round to 1: the derivative is the parameter
 // itself, with one of at most three logarithms, and a step is a multiplication, an addition and the exit test.  That is how
 // nearly every orbit of a frame over [0,4]^2 that ends does end (x runs down to zero where rA*rB < 1), a whole region's after
 // one another.
@@ -152,7 +149,7 @@ __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB,
     bool dead = false;
     int j = first;
     const int end = first + n;
-    if (ps->x < 0x1p-600 && rA <= 256.0 && rB <= 256.0) {
+    if (ps->x < 0x1p-740 && rA <= 256.0 && rB <= 256.0) {
         const unsigned codes = rC > 0.0 && rC <= 256.0 ? 3 : 2;   // parameters that may be used this way
         double x = ps->x, lyap = ps->lyap, zA = 0.0, zB = 0.0, zC = 0.0;
         if (ACC) {
@@ -184,6 +181,61 @@ __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB,
         j += m;
     }
     return dead;
+}
+
+// An orbit whose value at the end of a chunk is, bit for bit, the one a whole number of periods ago goes round the same values
+// for good (nothing else enters a step), and a stable one comes to that after some 36/|lambda| steps: on the 4096^2 frame of
+// "AABAB" 200 + 2000 41 % of all steps follow in warps all of whose orbits have.  They are not walked.  Measured, together with
+// the launch-wide queue of tiles, which such uneven tiles need (without it the first is 20.3 ms and the last 2.44): that frame
+// 31.3 -> 19.1 ms, 8192 x 4096 of "BBBBBBAAAAAA" 500 + 4000 over [3.4,4]x[2.5,3.4] 125 -> 69.9, 800 x 600 of "AB" 100 + 10000
+// over [0.01,3.99]^2 4.43 -> 1.56; 2048^2 over [3.9,4]^2, where no orbit comes into a cycle, 8.00 -> 8.15.
+//
+// The longest cycle whose logarithms are kept (640 bytes a thread of local memory), and the chunks after which another value of
+// the orbit becomes the reference, at first: cycles that do not go into a chunk are found when they go into up to that many.
+// (Rounding makes cycles of nine from cycles of three.)
+constexpr int kMaxCycle = 80, kRefChunks = 6;
+static_assert(kMaxCycle >= kMaxChunk && kMaxCycle % 4 == 0, "a cycle that goes into a chunk is never too long");
+
+// The last n steps of an orbit that has come back to an earlier value, from step `first` of a region whose selector words start
+// at `sel` and repeat every `period` steps: it goes round the same values for good, so the logarithms of one turn are taken and
+// the rest of the sum is added up from them.  False (and nothing done) when a turn has more than kMaxCycle steps.
+__device__ __noinline__ bool cycle_steps(PixelState* ps, double rA, double rB, double rC, const unsigned* sel, int wrap, int period,
+                                         int first, int n, unsigned lane_off) {
+    double z[kMaxCycle];
+    const double x0 = ps->x;
+    double x = x0, sum = 0.0, below = 0.0, above = 0.0;
+    int len = 0, zeros = 0, wi = (first / kStepsPerWord) % wrap, in_word = first & (kStepsPerWord - 1);
+    unsigned word = sel[wi] >> (2 * in_word);
+    do {
+        if (len + period > kMaxCycle) return false;
+        for (int k = 0; k < period; ++k, ++len) {
+            const unsigned code = word & 3u;
+            word >>= 2;
+            if (++in_word == kStepsPerWord) {
+                in_word = 0;
+                if (++wi == wrap) wi = 0;
+                word = sel[wi];
+            }
+            const double r = code == 0 ? rA : (code == 1 ? rB : rC);
+            const double d = half_derivative(r, x);
+            x = __dmul_rn(__dmul_rn(r, x), __dsub_rn(1.0, x));
+            double t = -0.0;   // a step whose derivative is zero (:71): adding it changes nothing, and no logarithm is -0
+            if (d > 0.0) t = log_fast(d, lane_off);
+            else ++zeros;
+            z[len] = t;
+            sum = __dadd_rn(sum, t);
+            below = sum < below ? sum : below;
+            above = sum > above ? sum : above;
+        }
+    } while (x != x0);
+    for (int k = len; k & 3; ++k) z[k] = -0.0;
+    ps->lyap = lyap_cycle_sum(z, len, below, above, ps->lyap, n);
+    ps->valid += n;
+    if (zeros) {
+        ps->valid -= zeros * (n / len);
+        for (int k = 0; k < n % len; ++k) ps->valid -= (unsigned long long)__double_as_longlong(z[k]) == 0x8000000000000000ull;
+    }
+    return true;
 }
 
 // U consecutive logistic steps of all P pixels, selector bits in `word` (step j at bits 2j, 2j+1).
@@ -309,18 +361,18 @@ __device__ __forceinline__ unsigned compress_even_bits(unsigned w) {
 // n steps of selector word `word` (2 bits per step: 0 = A, 1 = B, 2 = C).
 template <int P, bool ACC, bool HAS_C, int UNROLL>
 __device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], double rA, const double (&rB)[P], double rC, unsigned word, int n, unsigned lane_off) {
-    if (n == kStepsPerWord) {
-        constexpr int U = HAS_C ? 2 : UNROLL;
-        unsigned pat = HAS_C ? word : compress_even_bits(word);
-        constexpr int kBits = HAS_C ? 2 * U : U;
+    constexpr int U = HAS_C ? 2 : UNROLL;
+    unsigned pat = HAS_C ? word : compress_even_bits(word);
+    constexpr int kBits = HAS_C ? 2 * U : U;
+    const int pairs = n / U;
 #pragma unroll 1
-        for (int h = 0; h < kStepsPerWord / U; ++h) {
-            dispatch_group<P, ACC, HAS_C, U>(x, lyap, rA, rB, rC, pat & ((1u << kBits) - 1u), lane_off);
-            pat >>= kBits;
-        }
-    } else {
-#pragma unroll 1
-        for (int j = 0; j < n; ++j, word >>= 2) fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word, lane_off);
+    for (int h = 0; h < pairs; ++h) {
+        dispatch_group<P, ACC, HAS_C, U>(x, lyap, rA, rB, rC, pat & ((1u << kBits) - 1u), lane_off);
+        pat >>= kBits;
+    }
+    if (n % U) {
+        word >>= 2 * (n - 1);
+        fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word, lane_off);
     }
 }
 
@@ -354,6 +406,9 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
     const double rC = a.c_value;
     int valid[P];
     bool done[P], careful_only[P];
+    double ref[P];        // an earlier value of the orbit, from a step that is a multiple of the sequence's period ago
+    bool in_cycle[P], no_cycle[P];   // it has come back to one (and at every later test does); its cycle is too long
+    int ref_left = 1, ref_chunks = kRefChunks;   // chunks up to the next such value, and from it to the one after
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         rB[p] = __dadd_rn(a.min_y, __dmul_rn(a.dy, (double)(int)(a.row_begin + row + p)));       // :42
@@ -363,7 +418,48 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         lam[p] = -5.0;
         done[p] = !inside || rA <= 0.0 || rB[p] <= 0.0;                                           // :47-50
         careful_only[p] = !(ordinary_param(rA) && ordinary_param(rB[p]) && a.fast_ok_c);
+        ref[p] = 0.0;
+        in_cycle[p] = false;
+        no_cycle[p] = careful_only[p];
     }
+    // Behind every whole chunk of the accumulation, whose steps are a multiple of the period: the pixels whose orbit stands
+    // where it stood a chunk ago or at the reference value are in a cycle, and when all of the warp's are (or have ended), the
+    // `left` steps from `next` on are added up from one turn of each (cycle_steps).  Lanes that are in one before the others
+    // go on walking; refilling them with other pixels costs more in warm-ups run for a part of a warp than it saves.  The
+    // generic kernel has no registers left for the reference value (it spills: 1.02 -> 1.07 ms); its chunks hold cycles of
+    // three where they can.
+    auto cycles = [&](const double (&sx)[P], const unsigned* sel, int wrap, int period, int next, int left) {
+        bool all = true;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            in_cycle[p] = in_cycle[p] || x[p] == sx[p] || (KG > 0 && x[p] == ref[p]);
+            all = all && (done[p] || (in_cycle[p] && !no_cycle[p]));
+        }
+        if (KG > 0 && --ref_left == 0) {
+            ref_left = ref_chunks;
+            ref_chunks += ref_chunks / 2;
+#pragma unroll
+            for (int p = 0; p < P; ++p) ref[p] = x[p];
+        }
+        if (!__all_sync(0xFFFFFFFFu, all) || left < kMaxCycle) return;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            bool ended = false;
+            if (!done[p]) {
+                PixelState ps{x[p], lyap[p], valid[p]};
+                ended = cycle_steps(&ps, rA, rB[p], rC, sel, wrap, period, next, left, lane_off);
+                if (ended) {
+                    done[p] = true;
+                    lam[p] = ps.valid > 0 ? __ddiv_rn(ps.lyap, __dmul_rn((double)ps.valid, LYAP_LN2)) : -5.0;
+                    my_steps += (unsigned long long)left;
+                } else {
+                    no_cycle[p] = true;
+                }
+            }
+            const unsigned lanes = __ballot_sync(0xFFFFFFFFu, ended);
+            if (a.cycle_steps && lanes && (threadIdx.x & 31) == 0) atomicAdd(a.cycle_steps, (unsigned long long)left * __popc(lanes));
+        }
+    };
 
     for (int region = 0; region < 2; ++region) {
         const bool acc = region == 1;
@@ -372,8 +468,9 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         const int wrap = acc ? a.acc_wrap : a.wu_wrap;
         if constexpr (KG > 0) {
             // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
-            // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code)
-            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = 2, CS = CB * BS * REP;
+            // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code); three of
+            // 16 steps hold cycles of three too
+            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = CB * BS == kStepsPerWord ? 3 : 2, CS = CB * BS * REP;
             static_assert(CS <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
             const unsigned* sel = a.sel + word0;
             int s = 0;
@@ -434,22 +531,23 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
                         }
                     }
                 }
+                if (acc && n == CS) cycles(sx, sel, wrap, BS, s + n, nsteps - s - n);
                 s += n;
             }
             continue;
         }
-        // generic walk: the selector words one after the other, exit tests after every second full word
+        // generic walk: exit tests after every second selector word, or after a.acc_chunk steps of the accumulation
         static_assert(2 * kStepsPerWord <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
         const unsigned* sel = a.sel + word0;
-        int s = 0, wi = 0;
+        const int chunk = acc ? a.acc_chunk : 2 * kStepsPerWord;
+        int s = 0, wi = 0, in_word = 0;   // step s is step in_word of word wi
         while (s < nsteps) {
             bool all_done = true;
 #pragma unroll
             for (int p = 0; p < P; ++p) all_done = all_done && done[p];
             if (__all_sync(0xFFFFFFFFu, all_done)) break;
 
-            const int left = nsteps - s;
-            const int n = left >= 2 * kStepsPerWord ? 2 * kStepsPerWord : (left >= kStepsPerWord ? kStepsPerWord : left);
+            const int n = min(chunk, nsteps - s);
             double sx[P], sl[P];
 #pragma unroll
             for (int p = 0; p < P; ++p) {
@@ -458,9 +556,13 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             }
 #pragma unroll 1
             for (int k = 0; k < n; k += kStepsPerWord) {
-                const unsigned word = sel[wi];
-                if (++wi == wrap) wi = 0;
-                const int m = min(kStepsPerWord, n - k);
+                const int m = min(kStepsPerWord, n - k), after = wi + 1 == wrap ? 0 : wi + 1;
+                const unsigned word = __funnelshift_r(sel[wi], sel[after], 2 * in_word);
+                in_word += m;
+                if (in_word >= kStepsPerWord) {
+                    in_word -= kStepsPerWord;
+                    wi = after;
+                }
                 if (acc) fast_chunk<P, true, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
                 else fast_chunk<P, false, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
             }
@@ -486,6 +588,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
                     }
                 }
             }
+            if (acc && a.acc_period && n == chunk) cycles(sx, sel, wrap, a.acc_period, s + n, nsteps - s - n);
             s += n;
         }
     }
@@ -528,13 +631,12 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
         exp_tab[e] = v;
     }
     unsigned long long my_steps = 0;
-    // Work is dealt out to blocks round-robin (tile t to block t % gridDim), first a.wide_tiles warp-tiles of 32*P pixels,
-    // then the rest of the frame in tiles of 32 pixels; a block's tiles go round its four schedulers (a warp's scheduler is
-    // warp % 4), and a warp that is done takes its scheduler's next tile from a counter in shared memory.  Warps whose orbits
-    // leave (0,1) early so take more tiles, and the small ones at the end fill what the wide ones leave ragged: a scheduler's
-    // time is its pixels times a constant whatever its warps' shapes (2200 steps: 103 / 168 / 238 / 312 us for 1 / 2 / 3 / 4
-    // warps of 2 pixels a thread, 58 / 93 / 123 / 158 us for 1 / 2 / 3 / 4 of one).  With one counter a block the first
-    // scheduler to be done takes all small tiles of a frame of one round: 512 x 512 in 0.301 instead of 0.287 ms.
+    // Work is dealt out per warp: first a.wide_tiles warp-tiles of 32*P pixels, then the rest of the frame in tiles of 32 pixels
+    // (a scheduler's time is its pixels times a constant whatever its warps' shapes: 2200 steps take 103 / 168 / 238 / 312 us
+    // with 1 / 2 / 3 / 4 warps of 2 pixels a thread, 58 / 93 / 123 / 158 us with 1 / 2 / 3 / 4 of one).  A tile whose orbits end
+    // or come into cycles soon takes a tenth of another's time, so a warp that is done takes the next tile of the launch from
+    // a counter in device memory.  Without one (see a.queue) tile t goes to block t % gridDim, and the block's tiles go round
+    // its four schedulers (a warp's scheduler is warp % 4) through counters in shared memory.
     __shared__ unsigned next_unit[4];   // the first units are taken as unit == warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < 4) next_unit[threadIdx.x] = THREADS / 32 + threadIdx.x;
@@ -545,16 +647,14 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
     const long long rows = a.n_pixels / a.width, positions = rows / P * a.width;
     const long long first = a.wide_tiles * 32, left = positions - first;
     const long long narrow_pixels = a.n_pixels - first * P;
-    const long long wide_of_block = a.wide_tiles > blockIdx.x ? (a.wide_tiles - blockIdx.x - 1) / gridDim.x + 1 : 0;
-    for (unsigned unit = warp;;) {
-        if (unit < wide_of_block) {
-            const long long q = ((long long)unit * gridDim.x + blockIdx.x) * 32 + lane, group = q / a.width;
+    for (long long t = (long long)warp * gridDim.x + blockIdx.x;;) {
+        if (t < a.wide_tiles) {
+            const long long q = t * 32 + lane, group = q / a.width;
             exact_tile<P, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, group * P, (int)(q - group * a.width), true, out64, out32, lane_off,
                                                                 my_steps);
         } else {
-            const long long tile = ((unit - wide_of_block) * gridDim.x + blockIdx.x) * 32;
-            if (tile >= narrow_pixels) break;
-            const long long m = tile + lane;
+            const long long m = (t - a.wide_tiles) * 32 + lane;
+            if (m - lane >= narrow_pixels) break;
             long long row, col;
             if (m < left * P) {
                 const long long p = m / left, q = first + (m - p * left);
@@ -567,8 +667,15 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
             }
             exact_tile<1, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, row, (int)col, m < narrow_pixels, out64, out32, lane_off, my_steps);
         }
-        if (lane == 0) unit = atomicAdd(&next_unit[warp & 3], 4u);
+        unsigned unit = 0;
+        if (lane == 0) unit = a.queue ? atomicAdd(a.queue, 1u) : atomicAdd(&next_unit[warp & 3], 4u);
         unit = __shfl_sync(0xFFFFFFFFu, unit, 0);
+        t = a.queue ? unit + (long long)gridDim.x * (THREADS / 32) : (long long)unit * gridDim.x + blockIdx.x;
+    }
+    // the last warp to be done leaves the queue as it was found
+    if (a.queue && lane == 0 && atomicAdd(a.queue + 1, 1u) == gridDim.x * (THREADS / 32) - 1) {
+        a.queue[0] = 0;
+        a.queue[1] = 0;
     }
 
     if (steps_out) {

@@ -22,9 +22,9 @@ namespace lyap {
 
 // The wide tiles' shape.  2048 x 2048 of "AABAB" 200 + 2000 / "BBBBBBAAAAAA" 500 + 4000, frame 0 of the zoom (a third of its
 // orbits end) and the 800 x 800 page: 2 pixels a thread 7.92 / 15.75 / 4.48 / 0.676 ms, 3 pixels 7.90 / 15.96 / 4.66 / 0.716,
-// 3 pixels side by side in a row 7.84 / 15.80 / 4.90 / 0.705 (128 registers and a few spilled); 4 of 384 threads 8.00 / 16.9.
-// The generic kernel picks a straight-line body every two steps for all of a thread's pixels: 3 pixels 1.02 ms, 2 pixels 1.05
-// (1277 x 719, 37 letters, 100 + 1000).
+// 3 pixels side by side in a row 7.84 / 15.80 / 4.90 / 0.705 (128 registers and a few spilled); 4 of 384 threads 8.00 / 16.9
+// (all before cycles were cut short).  The generic kernel picks a straight-line body every two steps for all of a thread's
+// pixels: 3 pixels 1.02 ms, 2 pixels 1.07 (1277 x 719 over [3.8,4]^2, 37 letters, 100 + 1000).
 constexpr int kExactThreads = 512, kExactPixels = 2, kGenericPixels = 3;
 
 template <bool HAS_C>
@@ -50,15 +50,14 @@ static int spec_mode() {
     return (jit < 0 ? 0 : (jit > 2 ? 2 : jit)) | (pre ? kSpecUsePrebuilt : 0);
 }
 
-// Deals a launch out for wide tiles of `pixels` a thread: whole rounds of them over the device's schedulers (4 an SM); 2 to 5
-// tiles of 32 pixels a scheduler are left to even out the end, and what is left of the rows' groups.  Returns the grid: the
-// shared tables allow one CTA per SM.
-static unsigned deal_exact(LambdaArgs* a, int pixels, int sm_count) {
-    const long long wide_px = 32LL * pixels, schedulers = 4LL * sm_count;
-    const long long rounds = std::min((a->n_pixels - 64 * schedulers) / (wide_px * schedulers),
-                                      a->n_pixels / a->width / pixels * a->width / (32 * schedulers));
-    a->wide_tiles = rounds > 0 ? rounds * schedulers : 0;
-    const long long warp_tiles = a->wide_tiles + (a->n_pixels - a->wide_tiles * wide_px + 31) / 32;
+// Deals a launch out: wide tiles of `pixels` a thread first, then `narrow_rounds` tiles of 32 pixels a warp of the grid (and what
+// is left of the rows' groups), which even out the end.  Returns the grid: the shared tables allow one CTA per SM.
+static unsigned deal_exact(LambdaArgs* a, int pixels, int narrow_rounds, int sm_count) {
+    const long long warps = (long long)kExactThreads / 32 * sm_count;
+    const long long wide_px = a->n_pixels - narrow_rounds * 32 * warps;
+    const long long groups = a->n_pixels / a->width / pixels * a->width / 32;   // wide tiles in the rows' whole groups
+    a->wide_tiles = std::max(0LL, std::min(wide_px / (32 * pixels), groups));
+    const long long warp_tiles = a->wide_tiles + (a->n_pixels - a->wide_tiles * 32 * pixels + 31) / 32;
     return (unsigned)std::min<long long>(warp_tiles, sm_count);
 }
 
@@ -67,7 +66,12 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     if (args.n_pixels <= 0) return cudaSuccess;
     LambdaArgs a = args;
     // a periodic sequence can run an instance of this kernel made for its patterns
-    unsigned grid = deal_exact(&a, kExactPixels, sm_count);
+    // Frames of up to ten tiles of 32 a warp go in such tiles alone: with 1 / 2 / 4 / 8 / all rounds of them 800 x 800 of "AB"
+    // 100 + 1000 over [0.01,3.99]^2 takes 471 / 471 / 471 / 447 / 426 us and 512 x 512 over [2,4]^2 215 / 210 / 202 / 202 / 202;
+    // 1920 x 1080 of "ABC" 300 + 3000 3675 / 3694 / 3701 / 3717 / 3758.  The generic kernel's choice of a body serves all of a
+    // thread's pixels: 1277 x 719 of 37 letters 864 / 892 / 930 / 989 / 1028.
+    const long long warps = (long long)kExactThreads / 32 * sm_count;
+    unsigned grid = deal_exact(&a, kExactPixels, a.n_pixels <= 10 * 32 * warps ? 10 : 2, sm_count);
     bool launched = false;
     const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads, kExactSmemBytes,
                                              spec_mode(), &launched);
@@ -75,7 +79,7 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     bool has_c = false;
     const int words = a.acc_word0 + (a.iterations > 0 ? min(a.acc_wrap, (a.iterations - 1) / kStepsPerWord + 1) : 0);
     for (int i = 0; i < words; ++i) has_c = has_c || (a.sel[i] & 0xAAAAAAAAu);
-    grid = deal_exact(&a, kGenericPixels, sm_count);
+    grid = deal_exact(&a, kGenericPixels, 1, sm_count);
     return has_c ? launch_exact_generic<true>(a, out64, out32, steps, grid, st)
                  : launch_exact_generic<false>(a, out64, out32, steps, grid, st);
 }

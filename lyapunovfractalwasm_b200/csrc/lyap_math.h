@@ -122,6 +122,73 @@ LYAP_HD double lyap_log_tab(double d, const lyap_logtab_entry* tab, int stride) 
 static inline double lyap_log(double d) { return lyap_log_tab(d, lyap_logtab_host, 1); }
 #endif
 
+// s + z[0] + z[1] + ... + z[len - 1], len a multiple of 4
+LYAP_HD double lyap_add_turn(const double* z, int len, double s) {
+    for (int j = 0; j < len; j += 4) {
+        const double z0 = z[j], z1 = z[j + 1], z2 = z[j + 2], z3 = z[j + 3];
+        s = s + z0;
+        s = s + z1;
+        s = s + z2;
+        s = s + z3;
+    }
+    return s;
+}
+
+LYAP_HD uint32_t lyap_high_word(double x) {
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)__double2hiint(x);
+#else
+    return (uint32_t)(lyap_bits(x) >> 32);
+#endif
+}
+
+// s + z[0] + z[1] + ... , n additions one after the other, z starting over after its `len` <= 1024 terms: the bits of that loop,
+// most of whose turns are jumped over.  z is filled up with -0.0, which changes no sum, to a multiple of 4 terms; the sums of a
+// turn's first terms lie between below <= 0 and above >= 0, as far as sums of doubles say.
+// While the sums stay inside one binade [2^e, 2^(e+1)) they are whole multiples N of its last place u, and N + z/u is rounded
+// to a whole number: by the same amount whatever N is, or, where z/u is half a whole number, by one that only N's parity decides.
+// So when one turn (or two, where one turns the parity over) has ended on the parity it began with, every further one adds
+// the same, step for step, until a sum might leave the binade.
+LYAP_HD double lyap_cycle_sum(const double* z, int len, double below, double above, double s, int n) {
+    const int padded = (len + 3) & ~3;
+    int turns = n / len, unit = 0;   // turns to go, turns since s0
+    const int rest = n - turns * len;
+    below = -below;
+    const double slack = (above + below) * 0x1p-36;   // many times the rounding of a turn's sums and of the bounds, u itself included
+    double s0 = s;
+    while (turns > 0) {   // one place where turns are walked, so that the lanes of a warp walk theirs together
+        s = lyap_add_turn(z, padded, s);
+        --turns;
+        ++unit;
+        const uint64_t change = lyap_bits(s) ^ lyap_bits(s0);
+        if ((change & 1u) == 0 || unit == 2) {
+            if (change == 0) {   // nothing changes any more
+                turns &= unit - 1;
+            } else if ((change & 1u) == 0 && change >> 52 == 0 && turns >= unit) {
+                // the magnitudes that the sums have come to lie between, and the binade's end that they move towards
+                const bool negative = s < 0.0;
+                const double m0 = negative ? -s0 : s0, m = negative ? -s : s, loose = LYAP_FMA(m0, 0x1p-36, slack);
+                const double outer = LYAP_FMA((double)unit, (negative ? below : above) + loose, m0);
+                const double inner = LYAP_FMA((double)-unit, (negative ? above : below) + loose, m0);
+                const uint32_t field = lyap_high_word(outer) >> 20;
+                if (field == lyap_high_word(inner) >> 20 && field > 1023 - 60 && field < 1023 + 60) {
+                    const double base = lyap_from_bits((uint64_t)field << 52), d = m - m0;
+                    const double room = d > 0.0 ? LYAP_FMA(base, 2.0, -outer) : inner - base;
+                    const float most = (float)room / (float)(d < 0.0 ? -d : d) * 0.999999f;
+                    int jump = turns >> (unit - 1);
+                    if (most < (float)jump) jump = (int)most;
+                    s = LYAP_FMA((double)jump, negative ? -d : d, s);   // exact: a multiple of u inside the binade
+                    turns -= jump << (unit - 1);
+                }
+            }
+            s0 = s;
+            unit = 0;
+        }
+    }
+    for (int j = 0; j < rest; ++j) s = s + z[j];
+    return s;
+}
+
 // 2^n * p for p in [0.5, 4), any n: two-step scaling keeps subnormal results single-rounded enough
 // for our use (results below 2^-1022 are rounded twice; never reached by the colour path).
 LYAP_HD double lyap_scalbn_small(double p, int n) {

@@ -37,6 +37,17 @@
 extern "C" {
 
 double oracle_log(double x) { return lyap_log(x); }
+double oracle_cycle_sum(const double* terms, int len, double s, int n) {
+    std::vector<double> z(terms, terms + len);
+    double sum = 0.0, below = 0.0, above = 0.0;
+    for (double t : z) {
+        sum += t;
+        below = std::min(below, sum);
+        above = std::max(above, sum);
+    }
+    z.resize((len + 3) / 4 * 4, -0.0);
+    return lyap_cycle_sum(z.data(), len, below, above, s, n);
+}
 double oracle_exp(double x) { return lyap_exp(x); }
 double oracle_pow(double x, double y) { return lyap_pow(x, y); }
 double oracle_sin(double x) { return lyap_sin(x); }

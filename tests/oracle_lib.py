@@ -28,6 +28,8 @@ class Port:
         for n in ("oracle_log", "oracle_exp", "oracle_sin", "oracle_cos"):
             getattr(L, n).restype = ctypes.c_double
             getattr(L, n).argtypes = [ctypes.c_double]
+        L.oracle_cycle_sum.restype = ctypes.c_double
+        L.oracle_cycle_sum.argtypes = [c_double_p, ctypes.c_int, ctypes.c_double, ctypes.c_int]
         L.oracle_pow.restype = ctypes.c_double
         L.oracle_pow.argtypes = [ctypes.c_double, ctypes.c_double]
         L.oracle_hash64.restype = ctypes.c_uint64

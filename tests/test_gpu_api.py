@@ -457,3 +457,29 @@ def test_multi_object_on_distinct_devices_with_nccl(engine):
     # the one-call form over distinct devices
     multi = L.render_multi(L.make_params(**kw), list(range(n)))
     assert np.array_equal(multi["rgba"], one["rgba"]) and np.array_equal(multi["lambda"].view(np.uint64), one["lambda"].view(np.uint64))
+
+
+def test_a_captured_lambda_launch_shares_nothing_with_direct_ones(engine):
+    """Direct launches take their tiles from the context's queue; one captured in a graph may run beside them, and deals its own."""
+    import torch
+    kw = dict(min_x=0.5, max_x=4.0, min_y=0.5, max_y=4.0, width=1023, height=517, sequence="AB", iterations=500, warmup=50)
+    p = L.make_params(**kw)
+    n = kw["width"] * kw["height"]
+    want = engine.compute_fractal(p)
+    mine, other = torch.cuda.Stream(), torch.cuda.Stream()
+    captured, direct = (torch.zeros(n, dtype=torch.float64, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    engine.set_stream(mine.cuda_stream)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=mine, capture_error_mode="relaxed"):
+            engine.lambda_device(p, d_lambda=captured.data_ptr())
+        for _ in range(4):
+            with torch.cuda.stream(other):
+                graph.replay()
+            engine.lambda_device(p, d_lambda=direct.data_ptr())
+        torch.cuda.synchronize()
+    finally:
+        engine.set_stream(None)
+    for got in (captured, direct):
+        assert np.array_equal(got.cpu().numpy().view(np.uint64), want.ravel().view(np.uint64))

@@ -243,3 +243,41 @@ def test_seeded_random_cases_against_the_oracle(engine, port, kernel_path):
         assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps, kw
         norm = port.normalize(lam)
         assert same_bits(r["norm"], norm) and np.array_equal(r["rgba"], port.colorize(norm, case % 7)), kw
+
+
+CYCLE_CASES = [
+    # window, size, sequence, iterations, warm-up, c: what is at its edge
+    ((2.0, 3.9, 2.0, 3.9), (129, 61), "AB", 1000, 100, None),        # (2, 2): x = 1/2 for good, no term at all
+    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 79, 0, None),    # one step too few are left behind the ninth chunk
+    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 80, 0, None),    # just enough
+    ((2.5, 4.0, 2.5, 4.0), (131, 67), "AABAB", 2011, 200, None),     # whole and single steps behind the last chunk
+    ((3.4, 4.0, 2.5, 3.4), (97, 50), "BBBBBBAAAAAA", 4000, 500, None),
+    ((3.815, 3.825, 3.445, 3.455), (95, 40), "ABC", 3000, 300, 3.7),
+    ((3.835, 3.837, 3.835, 3.837), (120, 33), "A", 5000, 10, None),  # cycles of three, six and (rounding) nine
+    ((2.5, 4.0, 2.5, 4.0), (101, 57), "ABBABAABBBABAABABBBAABABAABBBABBAAABA", 3000, 100, None),
+    ((2.5, 4.0, 2.5, 4.0), (70, 31), "AB" * 19 + "BAB", 2000, 41, None),    # a period of 41: chunks of an odd number of steps
+    ((2.5, 4.0, 2.5, 4.0), (70, 31), "AB" * 39 + "BA", 2000, 0, None),      # 80 steps, the longest period that is looked for
+    ((2.5, 4.0, 2.5, 4.0), (70, 31), "AB" * 39 + "BAB", 2000, 3, None),     # 81: none is
+    ((2.5, 4.0, 2.5, 4.0), (70, 31), "ABBAB" * 8, 20000, 3, None),          # a shorter period inside, selectors wrapped
+    ((0.05, 4.0, 0.05, 4.0), (90, 70), "ABB", 1500, 150, None),      # exits and falls beside cycles
+]
+
+
+@pytest.mark.parametrize("generic", [False, True], ids=["instance", "generic"])
+@pytest.mark.parametrize("case", CYCLE_CASES, ids=lambda c: "%s_%d" % (c[2][:12], c[3]))
+def test_orbits_that_come_into_cycles(engine, port, monkeypatch, case, generic):
+    """What is taken from a cycle has the bits of the orbit walked to its end: lambda, the exits and the count of steps."""
+    window, (width, height), sequence, iterations, warmup, c = case
+    monkeypatch.setenv("LYAP_PREBUILT", "0" if generic else "1")
+    monkeypatch.setenv("LYAP_JIT", "0" if generic else "2")
+    kw = dict(min_x=window[0], max_x=window[1], min_y=window[2], max_y=window[3], width=width, height=height, sequence=sequence,
+              iterations=iterations, warmup=warmup, c=c)
+    before = engine.cycle_steps()
+    r = engine.render(L.make_params(**kw), want=("lambda",))
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam)
+    assert r["stats"].executed_steps == steps
+    taken = engine.cycle_steps() - before
+    assert 0 <= taken < steps
+    if len(sequence) < 80 and iterations > 1000 and not (generic and sequence == "A"):   # no chunk holds nine, and there is no reference value
+        assert taken > 0

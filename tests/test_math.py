@@ -2,10 +2,12 @@
 
 These functions define "bit-exact" for the engine (CPU oracle and CUDA kernels share them), so the
 test is about their quality, i.e. how far the engine can be from a libm-linked reference."""
+import ctypes
 import math
 import random
 
 import mpmath as mp
+import numpy as np
 import pytest
 
 mp.mp.prec = 200
@@ -79,3 +81,32 @@ def test_sin_cos_accuracy(port):
             wc = max(wc, ulps(L.oracle_cos(x), mp.cos(mp.mpf(x))))
     assert ws < 2.0 and wc < 2.0, (ws, wc)
     assert L.oracle_sin(0.0) == 0.0 and L.oracle_cos(0.0) == 1.0
+
+
+@pytest.mark.parametrize("kind", ["orbit", "ties", "tiny", "falling", "halves", "mixed"])
+def test_cycle_sum_has_the_bits_of_the_additions_one_by_one(port, kind):
+    """lyap_cycle_sum against the loop it stands for: terms that tie at the sum's last place, sums that rise or fall through
+    many binades, cross zero, start on a power of two or never change."""
+    rng = random.Random(kind)
+    for t in range(1500):
+        length = rng.randint(1, 6 if t % 3 else 80)
+        terms = [(rng.random() - 0.6) * 2.0 ** rng.randint(-2, 3) for _ in range(length)]
+        if kind == "ties":
+            terms = [math.ldexp(round(math.ldexp(v, 44)), -44) for v in terms]
+        elif kind == "tiny":
+            terms = [math.ldexp(rng.randint(-12, 4), -rng.randint(44, 47)) for _ in terms]
+        elif kind == "falling":
+            terms = [-abs(v) * 2.0 ** -rng.randint(0, 39) for v in terms]
+        elif kind == "halves":
+            terms = [0.5 * rng.randint(-2, 2) for _ in terms]
+        elif kind == "mixed":
+            terms = [v if rng.random() < 0.8 else -0.0 for v in terms]
+        start = (rng.random() - 0.5) * 2.0 ** rng.randint(-3, 10)
+        start = (start, 0.0, 2.0 ** rng.randint(-2, 7), -(2.0 ** rng.randint(0, 9)))[min(3, max(0, t % 16 - 12))]
+        n = rng.randint(0, 2500)
+        want = start
+        for k in range(n):
+            want = want + terms[k % length]
+        z = np.array(terms, dtype=np.float64)
+        got = port.lib.oracle_cycle_sum(z.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), length, start, n)
+        assert (got, math.copysign(1.0, got)) == (want, math.copysign(1.0, want)), (t, length, n, start.hex())
