@@ -50,14 +50,15 @@ static int spec_mode() {
     return (jit < 0 ? 0 : (jit > 2 ? 2 : jit)) | (pre ? kSpecUsePrebuilt : 0);
 }
 
-// Deals a launch out: wide tiles of `pixels` a thread first, then `narrow_rounds` tiles of 32 pixels a warp of the grid (and what
-// is left of the rows' groups), which even out the end.  Returns the grid: the shared tables allow one CTA per SM.
-static unsigned deal_exact(LambdaArgs* a, int pixels, int narrow_rounds, int sm_count) {
-    const long long warps = (long long)kExactThreads / 32 * sm_count;
-    const long long wide_px = a->n_pixels - narrow_rounds * 32 * warps;
+// Deals a launch out: wide tiles of `pixels` a thread first, then `narrow` tiles of 32 pixels a scheduler (and what is left of
+// the rows' groups), which even out the end.  With `rounds` or fewer tiles a warp the launch does without a queue.  Returns the
+// grid: the shared tables allow one CTA per SM.
+static unsigned deal_exact(LambdaArgs* a, int pixels, int narrow, int rounds, int sm_count) {
+    const long long wide_px = a->n_pixels - narrow * 32LL * 4 * sm_count;
     const long long groups = a->n_pixels / a->width / pixels * a->width / 32;   // wide tiles in the rows' whole groups
     a->wide_tiles = std::max(0LL, std::min(wide_px / (32 * pixels), groups));
     const long long warp_tiles = a->wide_tiles + (a->n_pixels - a->wide_tiles * 32 * pixels + 31) / 32;
+    if (warp_tiles <= (long long)rounds * kExactThreads / 32 * sm_count) a->queue = nullptr;
     return (unsigned)std::min<long long>(warp_tiles, sm_count);
 }
 
@@ -66,12 +67,15 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     if (args.n_pixels <= 0) return cudaSuccess;
     LambdaArgs a = args;
     // a periodic sequence can run an instance of this kernel made for its patterns
-    // Frames of up to ten tiles of 32 a warp go in such tiles alone: with 1 / 2 / 4 / 8 / all rounds of them 800 x 800 of "AB"
+    // Frames of up to 40 tiles of 32 a scheduler go in such tiles alone: with 4 / 8 / 16 / 32 / all of them 800 x 800 of "AB"
     // 100 + 1000 over [0.01,3.99]^2 takes 471 / 471 / 471 / 447 / 426 us and 512 x 512 over [2,4]^2 215 / 210 / 202 / 202 / 202;
     // 1920 x 1080 of "ABC" 300 + 3000 3675 / 3694 / 3701 / 3717 / 3758.  The generic kernel's choice of a body serves all of a
-    // thread's pixels: 1277 x 719 of 37 letters 864 / 892 / 930 / 989 / 1028.
-    const long long warps = (long long)kExactThreads / 32 * sm_count;
-    unsigned grid = deal_exact(&a, kExactPixels, a.n_pixels <= 10 * 32 * warps ? 10 : 2, sm_count);
+    // thread's pixels (1277 x 719 of 37 letters 864 / 892 / 930 / 989 / 1028), but fewer than six tiles a scheduler are better
+    // all small: 190 x 223 of "AABAB" 27 + 270 45 us, with some wide ones 73.
+    // Orbits of one length end on an SM's 16 warps at once, which then take 16 tiles from the queue where others get none: two
+    // rounds of tiles and fewer are dealt out beforehand (315 x 305 of "AB" 82 + 821 over [3.4,4]x[2.5,3.4]: 126 -> 104 us).
+    const int small = 40;
+    unsigned grid = deal_exact(&a, kExactPixels, a.n_pixels <= small * 32LL * 4 * sm_count ? small : 8, 2, sm_count);
     bool launched = false;
     const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads, kExactSmemBytes,
                                              spec_mode(), &launched);
@@ -79,7 +83,8 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     bool has_c = false;
     const int words = a.acc_word0 + (a.iterations > 0 ? min(a.acc_wrap, (a.iterations - 1) / kStepsPerWord + 1) : 0);
     for (int i = 0; i < words; ++i) has_c = has_c || (a.sel[i] & 0xAAAAAAAAu);
-    grid = deal_exact(&a, kGenericPixels, 1, sm_count);
+    a.queue = args.queue;
+    grid = deal_exact(&a, kGenericPixels, a.n_pixels <= 6 * 32LL * 4 * sm_count ? 6 : 4, 1, sm_count);
     return has_c ? launch_exact_generic<true>(a, out64, out32, steps, grid, st)
                  : launch_exact_generic<false>(a, out64, out32, steps, grid, st);
 }
