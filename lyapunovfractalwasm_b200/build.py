@@ -26,7 +26,7 @@ PREBUILT_SEQUENCES = [("AB", False, 100), ("AABAB", False, 200), ("BBBBBBAAAAAA"
                       ("ABB", False, 300)]
 # ... in the shapes the launchers ask for:
 # (kind: 0 exact / 1 fast fp64 / 2 fast fp32 / 3 fast fp64 on the exact orbit, pixels per thread, threads)
-PREBUILT_SHAPES = [(0, 2, 512), (1, 4, 512), (2, 2, 256), (3, 3, 512)]
+PREBUILT_SHAPES = [(0, 2, 512), (1, 2, 128), (2, 2, 128), (3, 2, 128)]
 NVRTC_OPTIONS = ["--gpu-architecture=sm_100a", "--fmad=false", "--std=c++17", "-lineinfo"]   # as csrc/lyap_jit.cu passes them
 
 

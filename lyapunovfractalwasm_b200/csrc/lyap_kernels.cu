@@ -995,50 +995,43 @@ cudaError_t launch_fp32_peak(float* sink, int sm_count, int iters, unsigned long
 namespace lyap {
 
 template <typename FL, int P>
-static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                        int sm_count, cudaStream_t st, int kind, int spec_ppt, int spec_threads,
+static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st, int kind, int spec_ppt, int spec_threads,
                                         const char* generic_name) {
+    if (a.n_pixels <= 0) return cudaSuccess;
+    // one tile of 32 * pixels a warp: blocks are many and small, so that the tiles, some of which take a tenth of others'
+    // time, are dealt out as SMs have room
+    const auto grid = [&](int pixels, int threads) {
+        const long long rows = a.n_pixels / a.width;   // the larger of the two ways to cut a frame (see lambda_fast_body)
+        const long long positions = std::max((rows + pixels - 1) / pixels * a.width, (a.n_pixels + pixels - 1) / pixels);
+        return (unsigned)((positions + threads - 1) / threads);
+    };
     {   // a periodic sequence can run an instance made for its patterns (same switches as the exact kernel)
         bool launched = false;
-        const long long px = (long long)spec_threads * spec_ppt, spec_tiles = (a.n_pixels + px - 1) / px;
-        const long long cap = 2048 / spec_threads * sm_count;
-        const unsigned spec_grid = (unsigned)(spec_tiles < cap ? spec_tiles : cap);
-        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, spec_grid, st, kind, spec_ppt, spec_threads, 0, spec_mode(),
-                                                 &launched);
-        if (e != cudaSuccess) return e;
-        if (launched) return cudaSuccess;
+        const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid(spec_ppt, spec_threads), st, kind, spec_ppt, spec_threads, 0,
+                                                 spec_mode(), &launched);
+        if (e != cudaSuccess || launched) return e;
     }
-    const long long tile_px = (long long)kFastThreads * P;
-    const long long tiles = (a.n_pixels + tile_px - 1) / tile_px;
-    if (tiles <= 0) return cudaSuccess;
-    int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lambda_fast<FL, P, kFastThreads>,
-                                                                  kFastThreads, 0);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    const long long cap = (long long)sm_count * per_sm;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    k_lambda_fast<FL, P, kFastThreads><<<grid, kFastThreads, 0, st>>>(a, out64, out32, steps);
+    k_lambda_fast<FL, P, kFastThreads><<<grid(P, kFastThreads), kFastThreads, 0, st>>>(a, out64, out32, steps);
     note_lambda_kernel(generic_name);
     return cudaGetLastError();
 }
 
-// measured best shapes for the instances made for a sequence: fused fp64 4 pixels/thread, same-orbit fp64 3, of 512 threads;
-// fp32 2 of 256: 4096 x 2048 pixels of "AABAB" 200 + 2000 take 2.54 / 2.58 ms with 512 / 256 threads, but 2048 x 2048 over
-// [0.01,3.99]^2, where a block waits for its slowest orbits, 2.34 / 2.04
+// Two pixels a thread, which come into cycles together more often than more do and leave registers for more warps: 2731 x 1537
+// of "ABB" 150 + 1500 over [2,4]^2 in fp64 with 4 / 3 / 2 pixels 1.10 / 0.97 / 0.94 ms, 4096^2 of "AABAB" 200 + 2000 in fp32 with
+// 4 / 2 pixels 3.95 / 3.40.
 cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                  int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<FusedF64, 4>(a, out64, out32, steps, sm_count, st, 1, 4, 512, "k_lambda_fast<FusedF64,4,256> (generic)");
+    return launch_lambda_fast_t<FusedF64, 2>(a, out64, out32, steps, st, 1, 2, 128, "k_lambda_fast<FusedF64,2,128> (generic)");
 }
 
 cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                  int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<FusedF32, 4>(a, out64, out32, steps, sm_count, st, 2, 2, 256, "k_lambda_fast<FusedF32,4,256> (generic)");
+    return launch_lambda_fast_t<FusedF32, 2>(a, out64, out32, steps, st, 2, 2, 128, "k_lambda_fast<FusedF32,2,128> (generic)");
 }
 
 cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                   int sm_count, cudaStream_t st) {
-    return launch_lambda_fast_t<OrbitF64, 4>(a, out64, out32, steps, sm_count, st, 3, 3, 512, "k_lambda_fast<OrbitF64,4,256> (generic)");
+    return launch_lambda_fast_t<OrbitF64, 2>(a, out64, out32, steps, st, 3, 2, 128, "k_lambda_fast<OrbitF64,2,128> (generic)");
 }
 
 }  // namespace lyap

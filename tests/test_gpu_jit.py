@@ -240,3 +240,23 @@ def test_fast_modes_on_falls_that_a_large_or_undefined_parameter_ends(engine, po
             r = engine.render(L.make_params(**k, mode=mode), want=("lambda",))
             assert r["stats"].executed_steps == steps, (mode, warmup)
             np.testing.assert_allclose(r["lambda"], want, rtol=0.0, atol=2.4e-11)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (1, 70), (70, 1), (31, 2), (33, 3), (64, 47)], ids=lambda s: "%dx%d" % s)
+@pytest.mark.parametrize("path", ["jit", "generic"])
+def test_fast_modes_on_orbits_that_come_into_cycles(engine, port, kernel_path, path, size):
+    """Turns of a cycle added up instead of walked, on both cuts of a frame into threads' pixels: the exits and the count of
+    steps are the restatement's, and lambda differs from its extended sum by the rounding of a factor a step (2^-24 or 2^-53 of
+    it, / ln 2 in the mean) and of a few operations at the end."""
+    kernel_path(path)
+    for sequence, iterations in (("AAB", 1000), ("AAB", 72 * 9), ("AB", 96 * 8 + 95), ("AB" * 18 + "A", 1500)):
+        kw = dict(min_x=2.1, max_x=3.0, min_y=2.2, max_y=3.4, width=size[0], height=size[1], sequence=sequence, iterations=iterations,
+                  warmup=33)
+        for mode, unit in ((L.MODE_FAST_FP64, 2.0 ** -53), (L.MODE_FAST_FP32, 2.0 ** -24)):
+            want, steps = port.fused_lambda(**kw, single=mode == L.MODE_FAST_FP32)
+            before = engine.cycle_steps()
+            r = engine.render(L.make_params(**kw, mode=mode), want=("lambda",))
+            assert r["stats"].executed_steps == steps
+            bound = 1.001 * unit / np.log(2.0) + 8 * 2.0 ** -53 * np.max(np.abs(want))
+            assert np.max(np.abs(r["lambda"] - want)) < bound, (sequence, iterations, mode)
+            assert size != (64, 47) or engine.cycle_steps() > before   # in the smaller frames a slow orbit holds every tile up
