@@ -19,7 +19,10 @@ Beside that headline the JSON line carries (unless --no-extras):
                 batch of zoom frames dealt round-robin (the other ranks wait on the host meanwhile)
 --config 3 / --config 4 make that frame the headline workload instead (strong scaling).
 
-Metric: logistic-map steps per second (executed steps of all ranks / max-over-ranks device time).
+Metric: logistic-map steps per second (the frame's steps up to the orbits' exits, as the reference performs and counts them,
+of all ranks / max-over-ranks device time).  The kernels do not walk an orbit that has come back to an earlier value any
+further: the rest of its sum is added up from one turn of its cycle, to the same bits.  `config` says how many of the steps
+were walked, `walked_steps_per_s` gives the rate of those alone, and `roofline` counts the instructions of those alone.
 `e2e` is the same metric through host buffers with every frame's outputs copied to pinned host memory inside the timed
 region, the copies of frame k overlapping the kernels of frame k + 1 (N = 1: one lyap_multi_render_frames call for the K
 frames; N > 1: the band path with two buffer sets); `e2e_blocking` (N = 1) is one blocking lyap_render call per frame.
@@ -343,6 +346,7 @@ def main():
             self.kernel_name = eng.lib.lyap_last_kernel().decode()
             barrier()
             self.d_steps.zero_()
+            cycled = eng.cycle_steps()
             self.lam_events, self.launches = [], 0
             sampler = ClockSampler(local_rank) if (sample_clocks and rank == 0) else None
             if sampler:
@@ -362,31 +366,32 @@ def main():
             ms = ev0.elapsed_time(ev1)
             ms_lambda = sum(a.elapsed_time(b) for a, b in self.lam_events) / len(self.lam_events)
             executed = int(self.d_steps.item()) * self.rows_own // self.rows_all     # halo rows excluded pro rata
+            cycled = (eng.cycle_steps() - cycled) * self.rows_own // self.rows_all   # of those, taken from cycles
             t = torch.tensor([ms, ms_lambda], dtype=torch.float64, device=dev)
-            s = torch.tensor([executed], dtype=torch.int64, device=dev)
+            s = torch.tensor([executed, cycled], dtype=torch.int64, device=dev)
             if dist is not None:
                 dist.all_reduce(t, op=dist.ReduceOp.MAX)
                 dist.all_reduce(s, op=dist.ReduceOp.SUM)
-            return {"ms": float(t[0]), "ms_lambda": float(t[1]), "executed": int(s[0]), "clocks": clocks,
+            return {"ms": float(t[0]), "ms_lambda": float(t[1]), "executed": int(s[0]), "cycled": int(s[1]), "clocks": clocks,
                     "launches": self.launches, "steps": steps}
 
         def pipe_numbers(self, m, peak64, peak32):
-            """Fractions of the pipe's issue rate and of its flop rate for the lambda kernel of measurement m."""
+            """Fractions of the pipe's issue rate and of its flop rate for the lambda kernel of measurement m: the instructions of
+            the steps that were walked (those taken from cycles are steps of the accumulation)."""
             kw, md = self.kw, self.kw.get("mode", L.MODE_EXACT)
             per_px_steps = kw["warmup"] + kw["iterations"]
             if md == L.MODE_EXACT:
-                ops = OPS_WARM * kw["warmup"] + OPS_ACC * kw["iterations"]
-                flops = FLOPS_WARM * kw["warmup"] + FLOPS_ACC * kw["iterations"]
+                ops, flops = (OPS_WARM, OPS_ACC), (FLOPS_WARM, FLOPS_ACC)
             elif md == L.MODE_FAST_FP64_ORBIT:      # the reference's 3 orbit operations; fma(-2,x,1) and the product when accumulating
-                ops = 3 * kw["warmup"] + 5 * kw["iterations"]
-                flops = 3 * kw["warmup"] + 6 * kw["iterations"]
+                ops, flops = (3, 5), (3, 6)
             else:
-                ops, flops = FAST_OPS * per_px_steps, FAST_FLOPS * per_px_steps
-            steps_per_launch = m["executed"] / m["steps"] / world * self.rows_all / self.rows_own   # one rank's launch, halo included
+                ops, flops = (FAST_OPS, FAST_OPS), (FAST_FLOPS, FAST_FLOPS)
+            per_launch = 1.0 / m["steps"] / world * self.rows_all / self.rows_own   # one rank's launch, halo included
+            executed, cycled = m["executed"] * per_launch, m["cycled"] * per_launch
             sec = m["ms_lambda"] * 1e-3
             peak = peak32 if md == L.MODE_FAST_FP32 else peak64
-            instr = steps_per_launch * ops / per_px_steps / sec
-            fl = steps_per_launch * flops / per_px_steps / sec
+            rate = lambda c: (executed * (c[0] * kw["warmup"] + c[1] * kw["iterations"]) / per_px_steps - cycled * c[1]) / sec
+            instr, fl = rate(ops), rate(flops)
             return {"achieved": instr / 1e12, "peak": peak / 1e12, "frac": instr / peak,
                     "achieved_tflops": fl / 1e12, "peak_tflops": 2 * peak / 1e12, "frac_flops": fl / (2 * peak)}
 
@@ -589,6 +594,7 @@ def main():
                           "caps frac_flops at 18/26 of frac",
             "peak_source": "measured in this run: independent FMA chains on all SMs (lyap_fp64_peak / lyap_fp32_peak); "
                            "MEASURED_PEAKS.json has no fp64/fp32 vector entry",
+            "counted": "instructions of the steps walked; what turning to a cycle and adding up its turns takes is not counted",
             "instr_per_step": {"warmup": OPS_WARM, "accumulated": OPS_ACC} if mode == L.MODE_EXACT else FAST_OPS,
             "flops_per_step": {"warmup": FLOPS_WARM, "accumulated": FLOPS_ACC} if mode == L.MODE_EXACT else FAST_FLOPS,
             "ms_per_launch": ms_lambda,
@@ -620,8 +626,10 @@ def main():
             "config": {"workload": workload,
                        "l2": "each step rewrites %.0f MiB of outputs per GPU (> 126 MB L2); the path has no input arrays"
                              % ((rows_all * width * 16 + rows_own * width * 4) / 2 ** 20),
+                       "walked_over_executed": 1.0 - m["cycled"] / max(1, m["executed"]),
                        "executed_over_nominal": executed_all / (args.steps * width * height * (kw["warmup"] + kw["iterations"]))},
             ("ms_per_frame" if strong else "ms_per_frame_4096"): ms / args.steps,
+            "walked_steps_per_s": (m["executed"] - m["cycled"]) / (m["ms"] * 1e-3),
             "roofline": roofline,
             "e2e": None if e2e_value is None else e2e_batch if (world == 1 and e2e_batch is not None) else
                    {"value": e2e_value, "unit": "steps/s", "h2d_bytes_per_step": ctypes.sizeof(L.LyapParams) + len(kw["sequence"]),
