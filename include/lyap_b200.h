@@ -297,7 +297,8 @@ int lyap_group_patterns(const lyap_params* params, int* groups, uint64_t* warmup
 /* ---- measurement ---- */
 
 /* *steps = how many of the executed steps of this context's lambda launches so far were taken from an orbit's cycle
- * instead of being walked (see lyap_lambda_device); waits for the context's stream. */
+ * instead of being walked (see lyap_lambda_device); waits for the context's stream.  Launches that were captured in a
+ * graph, and those on cudaStreamPerThread, are not counted. */
 int lyap_cycle_steps(lyap_ctx* ctx, uint64_t* steps);
 
 /* Issue-rate micro-benchmark of the fp64 pipe on the context's device: independent DFMA chains,

@@ -202,8 +202,8 @@ int build_args(const lyap_params* p, lyap::LambdaArgs* a, Geometry* g) {
 
 int launch_lambda(lyap_ctx* c, int mode, lyap::LambdaArgs& a, double* d64, float* d32, unsigned long long* steps) {
     Range range("lyap: lambda");
-    a.cycle_steps = ctx_cycle_steps(c);
     a.queue = queue_for_launch(c);
+    a.cycle_steps = a.queue ? ctx_cycle_steps(c) : nullptr;   // a graph may outlive the context: nothing of the context's goes in
     cudaError_t e;
     if (mode == LYAP_MODE_EXACT) e = lyap::launch_lambda_exact(a, d64, d32, steps, c->sm_count, c->stream);
     else if (mode == LYAP_MODE_FAST_FP64) e = lyap::launch_lambda_fast64(a, d64, d32, steps, c->sm_count, c->stream);
