@@ -190,7 +190,10 @@ int build_args(const lyap_params* p, lyap::LambdaArgs* a, Geometry* g) {
         // a fast mode's sum depends in its last digits on where an orbit is found to be in a cycle: the same steps as in an
         // instance made for the sequence
         const int bs = period % 2 ? 2 * period : period;
-        if (p->mode != LYAP_MODE_EXACT && bs <= 32) a->acc_chunk = lyap::fast_chunk(bs);
+        if (p->mode != LYAP_MODE_EXACT && bs <= 32) {
+            a->acc_chunk = lyap::fast_chunk(bs);
+            a->acc_period = lyap::fast_unit(bs);
+        }
     }
     const double c = p->c_value;
     a->fast_ok_c = (!seq_has_c || (c > 0x1p-20 && c < 0x1p20)) ? 1 : 0;

@@ -18,6 +18,8 @@ constexpr int kMaxChunk = 80;
 __host__ __device__ constexpr int fast_block_periods(int bs) { return (kStepsPerWord + bs - 1) / bs; }
 __host__ __device__ constexpr int fast_chunk_blocks(int bs) { return bs * fast_block_periods(bs) <= 20 && bs != 6 ? 6 : 4; }
 __host__ __device__ constexpr int fast_chunk(int bs) { return bs * fast_block_periods(bs) * fast_chunk_blocks(bs); }
+// Steps after which a turn of a cycle is looked at: whole periods, and some where they are short (a chunk is a multiple of it).
+__host__ __device__ constexpr int fast_unit(int bs) { return bs <= 4 ? 8 : bs; }
 constexpr int kMaxSelWords = 896;  // 14336 distinct steps through kernel parameters (kernel parameter space is 4 KB)
 
 struct LambdaArgs {
@@ -30,7 +32,7 @@ struct LambdaArgs {
     int acc_word0;
     int fast_ok_c;         // c_value is positive, finite and of ordinary magnitude (or unused)
     int wu_wrap, acc_wrap; // words after which each region's selectors repeat (>= the region's words when it is stored whole)
-    int acc_period;        // steps after which the accumulation's selectors repeat, 0 when that is more than kMaxChunk
+    int acc_period;        // steps after which the accumulation's selectors repeat (a fast mode's are whole units), 0 when that is more than kMaxChunk
     int acc_chunk;         // steps between two exit tests of the generic kernels: a multiple of acc_period, if there is one
     unsigned* queue;       // exact kernel: tiles handed out so far and warps that are done, both zero between launches; null: no queue
     unsigned long long* cycle_steps;   // counts steps taken from an orbit's cycle instead of being walked (may be null)

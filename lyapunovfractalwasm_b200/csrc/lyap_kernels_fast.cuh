@@ -206,12 +206,12 @@ struct LongProduct {
         e += field - 1023;
     }
     template <int KG, unsigned long long PATS, int J = 0>
-    __device__ __forceinline__ void period(T& x, T rA, T rB, T rC) {
-        if constexpr (J < 2 * KG) {
-            constexpr unsigned code = (unsigned)(PATS >> (2 * J)) & 3u;
+    __device__ __forceinline__ void unit(T& x, T rA, T rB, T rC) {
+        if constexpr (J < fast_unit(2 * KG)) {
+            constexpr unsigned code = (unsigned)(PATS >> (2 * (J % (2 * KG)))) & 3u;
             step(x, code == 0 ? rA : (code == 1 ? rB : rC));
-            if (J % kRun == kRun - 1 || J == 2 * KG - 1) strip();
-            period<KG, PATS, J + 1>(x, rA, rB, rC);
+            if (J % kRun == kRun - 1 || J == fast_unit(2 * KG) - 1) strip();
+            unit<KG, PATS, J + 1>(x, rA, rB, rC);
         }
     }
     // `times` times its logarithm but for the 2^e, which is had in two doubles: `times` is many and would multiply the
@@ -236,7 +236,7 @@ struct LongProduct {
 template <typename FL, bool ACC>
 __device__ __forceinline__ bool fast_careful_body(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                   typename FL::real rC, unsigned word, int n, LongProduct<FL>& product,
-                                                  unsigned long long* steps) {
+                                                  unsigned* steps) {
     using T = typename FL::real;
     using F = FastTraits<T>;
     T x = ps->x;
@@ -262,7 +262,7 @@ __device__ __forceinline__ bool fast_careful_body(FastPixel<typename FL::real>* 
         dead = !(x > (T)0 && x < (T)1);
     }
     product.strip();
-    *steps += (unsigned long long)j;
+    *steps += j;
     ps->x = x;
     ps->valid = valid;
     return dead;
@@ -273,7 +273,7 @@ __device__ __forceinline__ bool fast_careful_body(FastPixel<typename FL::real>* 
 template <typename FL, bool ACC>
 __device__ __forceinline__ int fast_fall(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                          typename FL::real rC, const unsigned* sel, int wrap, int first, int end,
-                                         unsigned long long* steps) {
+                                         unsigned* steps) {
     using T = typename FL::real;
     Fall<T, ACC> fall(rA, rB, rC);
     T x = ps->x;
@@ -286,7 +286,7 @@ __device__ __forceinline__ int fast_fall(FastPixel<typename FL::real>* ps, typen
         ps->valid += j - first;
         ps->extra = __dadd_rn(ps->extra, fall.sum());
     }
-    *steps += (unsigned long long)(j - first);
+    *steps += j - first;
     ps->x = x;
     return j;
 }
@@ -309,7 +309,7 @@ __device__ __forceinline__ void fast_mode_steps(typename FL::real (&x)[P], typen
 template <typename FL, bool ACC>
 __device__ __noinline__ bool fast_careful_steps(FastPixel<typename FL::real>* ps, typename FL::real rA, typename FL::real rB,
                                                 typename FL::real rC, const unsigned* sel, int wrap, int first, int n,
-                                                unsigned long long* steps) {
+                                                unsigned* steps) {
     using T = typename FL::real;
     LongProduct<FL> product;
     bool dead = false;
@@ -427,29 +427,41 @@ __device__ __forceinline__ void fast_word(typename FL::real (&x)[P], typename FL
     }
 }
 
+// Whole chunks that have to be left behind the one in which an orbit is found in a cycle.  Warps in which other orbits are not walk
+// on and walk a turn at the end besides: 276 x 283 of "AB" 23 + 238 over [3.9,4]^2 in fp32 takes 31.1 us without such a limit (and
+// with one), 20.9 with two or more; 3889 x 4085 of "ABBBBBBABA" 71 + 719 over [2.5,4]^2 in fp64 4.19 ms with two, 4.50 with four.
+constexpr int kLeastChunks = 3;
+
 // q times the sum of the logarithms of the derivatives (same orbit: of the factors |1 - 2x|) over n steps, whole periods, of an
-// orbit that stands at x again after them, none of them zero: one turn of its cycle is walked, from step `first` of a region
-// whose selector words start at `sel` (generic kernel) or from a period's start.  The sum is *exponent * log 2 + the result.
+// orbit that stands at x again after them, none of them zero: one turn of its cycle, in units of whole periods, is walked, from
+// step `first` of a region whose selector words start at `sel` (generic kernel) or from a period's start.  The sum is
+// *exponent * log 2 + the result.
 template <typename FL, int KG, unsigned long long PATS>
 __device__ __noinline__ double fast_cycle(typename FL::real x, typename FL::real rA, typename FL::real rB, typename FL::real rC,
-                                          const unsigned* sel, int wrap, int first, int period, int n, int q, int* exponent) {
+                                          const unsigned* sel, int wrap, int first, int unit, int n, int q, int* exponent) {
     using T = typename FL::real;
     const T x0 = x;
     LongProduct<FL> product;
     int len = 0;
     if constexpr (KG > 0) {
         do {
-            product.template period<KG, PATS>(x, rA, rB, rC);
-            len += 2 * KG;
+            product.template unit<KG, PATS>(x, rA, rB, rC);
+            len += fast_unit(2 * KG);
         } while (x != x0 && len < n);
     } else {
+        const unsigned head = selectors_from(sel, wrap, first);
         do {
-            for (int k = 0; k < period; ++k, ++len) {
-                const int j = first + len;
-                const unsigned code = (sel[(j / kStepsPerWord) % wrap] >> (2 * (j & (kStepsPerWord - 1)))) & 3u;
-                product.step(x, code == 0 ? rA : (code == 1 ? rB : rC));
-                if (k % LongProduct<FL>::kRun == LongProduct<FL>::kRun - 1 || k == period - 1) product.strip();
+            for (int k = 0; k < unit; k += kStepsPerWord) {
+                unsigned word = k == 0 ? head : selectors_from(sel, wrap, first + k);
+                const int m = min(kStepsPerWord, unit - k);
+                for (int j = 0; j < m; ++j, word >>= 2) {
+                    const unsigned code = word & 3u;
+                    product.step(x, code == 0 ? rA : (code == 1 ? rB : rC));
+                    if (j == LongProduct<FL>::kRun - 1) product.strip();
+                }
+                product.strip();
             }
+            len += unit;
         } while (x != x0 && len < n);
     }
     const int times = q * (n / len);
@@ -465,7 +477,7 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
     using T = typename FL::real;
     using F = FastTraits<T>;
     constexpr T kSign = FL::packed ? (T)-1 : (T)1;   // x[] holds kSign * x
-    unsigned long long my_steps = 0, cycle_steps = 0;
+    unsigned my_steps = 0, cycle_steps = 0;   // of a thread's pixels: no more than P * 2^24, and a warp's 2^30
     // A tile is 32 neighbouring positions.  In a frame of rows enough a position is a column of a group of P rows, whose
     // pixels lie below one another: tiles as high as they are compact come into cycles or leave (0,1) as a whole most often.
     // Where the last group would be mostly empty, the frame is one long row cut into P pieces, a pixel of each a position.
@@ -478,7 +490,10 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
     double extra[P];
     int valid[P], esum[P];   // 32 bits are enough: the host admits at most 2^24 steps per pixel in the fast modes
     int nuse[P][3];          // same-orbit flavour: accumulated steps of accepted chunks by the parameter they used (A, B, C)
-    bool done[P], careful_only[P], in_cycle[P];
+    // a pixel's state: on its way, on its way but step by step (an odd parameter), ended, or, from 0 on, the accumulated steps
+    // after which its orbit stood where it had stood a chunk before
+    constexpr int kWalks = -1, kCareful = -2, kDone = -3;
+    int state[P];
     // pixel p's place in the launch, or -1 where there is none
     auto place = [&](int p) -> long long {
         const long long group = at / a.width;
@@ -507,10 +522,9 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
         valid[p] = 0;
         esum[p] = 0;
         if constexpr (FL::same_orbit) nuse[p][0] = nuse[p][1] = nuse[p][2] = 0;
-        done[p] = i < 0 || ra <= 0.0 || rb <= 0.0;
-        careful_only[p] = !(ordinary_param_t<T>(rA[p]) && ordinary_param_t<T>(rB[p]) && a.fast_ok_c);
-        in_cycle[p] = false;
-        if (i >= 0 && done[p]) store(p, -5.0);
+        state[p] = ordinary_param_t<T>(rA[p]) && ordinary_param_t<T>(rB[p]) && a.fast_ok_c ? kWalks : kCareful;
+        if (i < 0 || ra <= 0.0 || rb <= 0.0) state[p] = kDone;
+        if (i >= 0 && state[p] == kDone) store(p, -5.0);
     }
 
     // lambda from the partial sums: esum*ln2 + log(mantissa product) + logarithms of falls, redone chunks and turns of a cycle
@@ -535,12 +549,13 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
         const unsigned* sel = a.sel + word0;
         // an instance's chunk: REP straight-line blocks of CB whole periods
         constexpr int BS = KG > 0 ? 2 * KG : 1, CB = fast_block_periods(BS), REP = fast_chunk_blocks(BS);
-        const int chunk = KG > 0 ? CB * BS * REP : a.acc_chunk, period = KG > 0 ? BS : a.acc_period;
+        const int chunk = KG > 0 ? CB * BS * REP : a.acc_chunk, unit = KG > 0 ? fast_unit(BS) : a.acc_period;
+        const int whole = acc && unit > 0 ? nsteps / chunk * chunk : 0;   // the steps in chunks that are a multiple of the period
         int s = 0;
         while (s < nsteps) {
             bool all_done = true;
 #pragma unroll
-            for (int p = 0; p < P; ++p) all_done = all_done && done[p];
+            for (int p = 0; p < P; ++p) all_done = all_done && state[p] == kDone;
             if (__all_sync(0xFFFFFFFFu, all_done)) break;
             const int left = nsteps - s;
             int n = min(left, chunk);
@@ -605,9 +620,14 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
             bool all_cycle = true;
 #pragma unroll
             for (int p = 0; p < P; ++p) {
-                if (done[p]) continue;
+                if (state[p] == kDone) continue;
+                if (state[p] >= 0) {   // sums stay as they were when it turned; x comes back by itself
+                    prod[p] = sp[p];
+                    esum[p] = se[p];
+                    continue;
+                }
                 // a zero derivative (or a product that underflowed) shows as exponent field 0
-                const bool regular = !careful_only[p] && (kSign * x[p] > (T)0 && kSign * x[p] < (T)1) && (!acc || emin[p] != 0);
+                const bool regular = state[p] == kWalks && (kSign * x[p] > (T)0 && kSign * x[p] < (T)1) && (!acc || emin[p] != 0);
                 if (regular) {
                     if (acc) {
                         valid[p] += n;
@@ -617,9 +637,9 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                             nuse[p][1] += cuse[1];
                             nuse[p][2] += cuse[2];
                         }
-                        in_cycle[p] = in_cycle[p] || (n == chunk && x[p] == sx[p]);
+                        if (s < whole - kLeastChunks * chunk && x[p] == sx[p]) state[p] = s + n;
                     }
-                    my_steps += (unsigned long long)n;
+                    my_steps += n;
                 } else {
                     prod[p] = sp[p];
                     FastPixel<T> ps{kSign * sx[p], extra[p], se[p], valid[p]};
@@ -631,53 +651,54 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                     valid[p] = ps.valid;
                     if (dead) {
                         // the result stands now: the abandoned lane keeps running on garbage
-                        done[p] = true;
+                        state[p] = kDone;
                         store(p, finish(p));
                         x[p] = kSign * (T)0.25;
                     }
                 }
-                all_cycle = all_cycle && (done[p] || in_cycle[p]);
+                all_cycle = all_cycle && (state[p] >= 0 || state[p] == kDone);
             }
             s += n;
-            // Behind a whole chunk, whose steps are a multiple of the period: when every orbit of the warp that is left has come
-            // back to the value it had a chunk before (as it will from then on), the whole chunks that are left are added
-            // up from one turn of its cycle.  4096^2 of "AABAB" 200 + 2000: fp32 4.75 -> 3.12 ms, fp64 8.37 -> 5.54, on the exact
-            // orbit 10.3 -> 6.9; 2731 x 1537 of "ABB" 150 + 1500 over [2,4]^2, fp64: 1.60 -> 0.90.
-            const int q = acc && n == chunk && period > 0 ? (nsteps - s) / chunk : 0;
-            if (q > 0 && __all_sync(0xFFFFFFFFu, all_cycle)) {
+            // An orbit that has come back to the value it had a chunk before (as it will from then on) leaves its sums as they
+            // are there, and the whole chunks that are left are added up from one turn of its cycle: a pixel's bits are its own,
+            // whichever others are in its warp, which walks on until all its orbits have, or to the last whole chunk's end.
+            // Cycles walked in full / this: 4096^2 of "AABAB" 200 + 2000 fp32 4.77 / 3.27 ms, fp64 8.37 / 5.65, on the exact orbit
+            // 10.4 / 7.02; 2731 x 1537 of "ABB" 150 + 1500 over [2,4]^2, fp64: 1.61 / 0.91.
+            if (s > whole || (s < whole && !__all_sync(0xFFFFFFFFu, all_cycle))) continue;
 #pragma unroll
-                for (int p = 0; p < P; ++p) {
-                    if (done[p]) continue;
-                    int exponent;
-                    extra[p] = __dadd_rn(extra[p], fast_cycle<FL, KG, ACC_PATS>(kSign * x[p], rA[p], rB[p], rC[p], sel, wrap, s, period,
-                                                                                 chunk, q, &exponent));
-                    esum[p] += exponent;
-                    valid[p] += q * chunk;
-                    if constexpr (FL::same_orbit) {
-                        nuse[p][0] += q * cuse[0];
-                        nuse[p][1] += q * cuse[1];
-                        nuse[p][2] += q * cuse[2];
-                    }
-                    cycle_steps += (unsigned long long)(q * chunk);
+            for (int p = 0; p < P; ++p) {
+                if (state[p] < 0) continue;
+                const int q = (whole - state[p]) / chunk;
+                int exponent;
+                extra[p] = __dadd_rn(extra[p], fast_cycle<FL, KG, ACC_PATS>(kSign * x[p], rA[p], rB[p], rC[p], sel, wrap, s, unit, chunk,
+                                                                             q, &exponent));
+                esum[p] += exponent;
+                valid[p] += q * chunk;
+                if constexpr (FL::same_orbit) {
+                    nuse[p][0] += q * cuse[0];
+                    nuse[p][1] += q * cuse[1];
+                    nuse[p][2] += q * cuse[2];
                 }
-                s += q * chunk;
+                my_steps += q * chunk;
+                cycle_steps += whole - s;
+                state[p] = kWalks;
             }
+            s = whole;
         }
     }
 
 #pragma unroll
     for (int p = 0; p < P; ++p) {
-        if (!done[p]) store(p, finish(p));
+        if (state[p] != kDone) store(p, finish(p));
     }
-    my_steps += cycle_steps;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         my_steps += __shfl_down_sync(0xFFFFFFFFu, my_steps, o);
         cycle_steps += __shfl_down_sync(0xFFFFFFFFu, cycle_steps, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        if (steps_out && my_steps) atomicAdd(steps_out, my_steps);
-        if (a.cycle_steps && cycle_steps) atomicAdd(a.cycle_steps, cycle_steps);
+        if (steps_out && my_steps) atomicAdd(steps_out, (unsigned long long)my_steps);
+        if (a.cycle_steps && cycle_steps) atomicAdd(a.cycle_steps, (unsigned long long)cycle_steps);
     }
 }
 

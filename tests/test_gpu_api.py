@@ -101,6 +101,31 @@ def test_progress_callback_is_ordered_and_ends_with_one(engine, port):
     assert np.array_equal(lam.view(np.uint64), again.view(np.uint64))
 
 
+@pytest.mark.parametrize("path", ["prebuilt", "generic"])
+@pytest.mark.parametrize("mode", [L.MODE_FAST_FP64, L.MODE_FAST_FP32, L.MODE_FAST_FP64_ORBIT])
+def test_fast_modes_however_a_frame_is_launched(engine, kernel_path, mode, path):
+    """A pixel's bits are its own: no matter which others are launched with it, or lie in its warp.  Bands that begin on an odd
+    row, single rows, several devices' bands with their halo rows, and the row chunks of a progress callback, at widths that
+    are no multiple of a warp, over a window with cycles, chaos and exits side by side."""
+    kernel_path(path)
+    kw = dict(min_x=1.9, max_x=4.0, min_y=2.1, max_y=4.0, width=77, height=61, sequence="AABAB", iterations=1500, warmup=200, mode=mode)
+    one = engine.render(L.make_params(**kw), want=("lambda", "norm", "rgba"))
+    whole = one["lambda"].view(np.uint64)
+    for y0, y1 in ((0, 13), (13, 14), (14, 47), (47, 48), (48, 61)):
+        band = engine.compute_fractal(L.make_params(**kw, row_begin=y0, row_end=y1))
+        assert np.array_equal(band.view(np.uint64), whole[y0:y1]), (y0, y1)
+    with L.Multi([0, 0, 0]) as m:
+        got = m.render(L.make_params(**kw), want=("lambda", "norm", "rgba"))
+    assert np.array_equal(got["lambda"].view(np.uint64), whole)
+    assert np.array_equal(got["norm"].view(np.uint64), one["norm"].view(np.uint64)) and np.array_equal(got["rgba"], one["rgba"])
+
+    kw.update(width=1531, height=1601, sequence="AB", iterations=700, warmup=100)
+    seen = []
+    chunks = engine.compute_fractal(L.make_params(**kw), progress=seen.append)
+    assert len(seen) >= 2
+    assert np.array_equal(chunks.view(np.uint64), engine.compute_fractal(L.make_params(**kw)).view(np.uint64))
+
+
 def test_fast_modes_within_stated_tolerance(engine):
     """Fast modes against exact on the config-1 frame.  Stated bounds: fp64 fast mode keeps 99% of the
     stable pixels (lambda < 0, > -4) within 1e-6 relative; fp32 fast mode keeps their median within 1e-5
