@@ -11,6 +11,8 @@ namespace lyap {
 constexpr int kStepsPerWord = 16;
 // Most steps between two exit tests of the exact kernels.
 constexpr int kMaxChunk = 80;
+// Steps that have to be left for the exact kernels' turning to an orbit's cycle to pay.
+constexpr int kLeastLeft = 160;
 // The fast kernels' chunk for a sequence whose pairs of steps repeat every `bs` steps: blocks of whole periods and at least 16
 // steps, so many of them that cycles of two, three, four and eight periods go into a chunk as far as 130 steps can hold them.
 // An exit test costs more the shorter the chunk is, a cycle is found the later the longer it is: 4096^2 of "AABAB" 200 + 2000

@@ -215,7 +215,6 @@ __device__ __noinline__ bool careful_steps(PixelState* ps, double rA, double rB,
 // the orbit becomes the reference, at first: cycles that do not go into a chunk are found when they go into up to that many.
 // (Rounding makes cycles of nine from cycles of three.)
 constexpr int kMaxCycle = 80, kRefChunks = 6;
-constexpr int kLeastLeft = 160;   // steps that have to be left for turning to the cycles to pay
 static_assert(kMaxCycle >= kMaxChunk && kMaxCycle % 4 == 0 && kLeastLeft >= kMaxCycle, "a cycle that goes into a chunk is never too long");
 
 // The last n steps of an orbit that has come back to an earlier value, from step `first` of a region whose selector words start
@@ -386,16 +385,14 @@ __device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], do
     constexpr int U = HAS_C ? 2 : UNROLL;
     unsigned pat = HAS_C ? word : compress_even_bits(word);
     constexpr int kBits = HAS_C ? 2 * U : U;
-    const int pairs = n / U;
+    int left = n;
 #pragma unroll 1
-    for (int h = 0; h < pairs; ++h) {
+    for (; left >= U; left -= U) {
         dispatch_group<P, ACC, HAS_C, U>(x, lyap, rA, rB, rC, pat & ((1u << kBits) - 1u), lane_off);
         pat >>= kBits;
     }
-    if (n % U) {
-        word >>= 2 * (n - 1);
-        fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word, lane_off);
-    }
+#pragma unroll 1
+    for (; left > 0; --left) fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word >> (2 * (n - left)), lane_off);
 }
 
 // ---- run-time specialisation -------------------------------------------------------------------
@@ -495,8 +492,9 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         if constexpr (KG > 0) {
             // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
             // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code); three of
-            // 16 steps hold cycles of three too
-            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = CB * BS == kStepsPerWord ? 3 : 2, CS = CB * BS * REP;
+            // 16 steps hold cycles of three too.  A warp of small tiles that is alone on its scheduler waits some 250 cycles behind
+            // every chunk: four blocks there (128 x 96 of "AABAB" 100 + 4000 over [3.9,4]^2 126 -> 112 us).
+            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = CB * BS == kStepsPerWord ? 3 : (P == 1 && CB * BS <= 20 ? 4 : 2), CS = CB * BS * REP;
             static_assert(CS <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
             const unsigned* sel = a.sel + word0;
             int s = 0;
@@ -568,7 +566,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         static_assert(2 * kStepsPerWord <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
         const unsigned* sel = a.sel + word0;
         const int chunk = acc ? a.acc_chunk : 2 * kStepsPerWord;
-        int s = 0, wi = 0, in_word = 0;   // step s is step in_word of word wi
+        int s = 0, wi = 0;
         while (s < nsteps) {
             bool all_done = true;
 #pragma unroll
@@ -576,6 +574,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             if (__all_sync(0xFFFFFFFFu, all_done)) break;
 
             const int n = min(chunk, nsteps - s);
+            if (acc && a.acc_period) wi = 0;   // whole periods lie behind: this chunk has the selectors of the first
             double sx[P], sl[P];
 #pragma unroll
             for (int p = 0; p < P; ++p) {
@@ -584,13 +583,9 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             }
 #pragma unroll 1
             for (int k = 0; k < n; k += kStepsPerWord) {
-                const int m = min(kStepsPerWord, n - k), after = wi + 1 == wrap ? 0 : wi + 1;
-                const unsigned word = __funnelshift_r(sel[wi], sel[after], 2 * in_word);
-                in_word += m;
-                if (in_word >= kStepsPerWord) {
-                    in_word -= kStepsPerWord;
-                    wi = after;
-                }
+                const int m = min(kStepsPerWord, n - k);
+                const unsigned word = sel[wi];
+                if (++wi == wrap) wi = 0;
                 if (acc) fast_chunk<P, true, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
                 else fast_chunk<P, false, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
             }
@@ -678,7 +673,7 @@ __device__ __forceinline__ void lambda_exact_body(const LambdaArgs& a, double* _
     const long long first = a.wide_tiles * 32, left = positions - first;
     const long long narrow_pixels = a.n_pixels - first * P;
     for (long long t = (long long)warp * gridDim.x + blockIdx.x;;) {
-        if (t < a.wide_tiles) {
+        if (P > 1 && t < a.wide_tiles) {
             const long long q = t * 32 + lane, group = q / a.width;
             exact_tile<P, HAS_C, UNROLL, KG, WU_PATS, ACC_PATS>(a, group * P, (int)(q - group * a.width), true, out64, out32, lane_off,
                                                                 my_steps);

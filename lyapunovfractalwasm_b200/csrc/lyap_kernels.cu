@@ -27,16 +27,17 @@ namespace lyap {
 // pixels: 3 pixels 1.02 ms, 2 pixels 1.07 (1277 x 719 over [3.8,4]^2, 37 letters, 100 + 1000).
 constexpr int kExactThreads = 512, kExactPixels = 2, kGenericPixels = 3;
 
-template <bool HAS_C>
+template <int P, bool HAS_C, int UNROLL>
 static cudaError_t launch_exact_generic(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                         unsigned grid, cudaStream_t st) {
-    auto kern = k_lambda_exact<kGenericPixels, kExactThreads, HAS_C, 2>;
+    auto kern = k_lambda_exact<P, kExactThreads, HAS_C, UNROLL>;
     constexpr size_t smem = kExactSmemBytes;
     // the attribute is per device and cheap to set; doing it on every launch keeps this thread- and device-safe
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     kern<<<grid, kExactThreads, smem, st>>>(a, out64, out32, steps);
-    note_lambda_kernel("k_lambda_exact<3,512> (generic: patterns dispatched every 2 steps)");
+    note_lambda_kernel(P == 1 ? "k_lambda_exact<1,512> (generic: patterns dispatched every 4 steps)"
+                              : "k_lambda_exact<3,512> (generic: patterns dispatched every 2 steps)");
     return cudaGetLastError();
 }
 
@@ -50,13 +51,12 @@ static int spec_mode() {
     return (jit < 0 ? 0 : (jit > 2 ? 2 : jit)) | (pre ? kSpecUsePrebuilt : 0);
 }
 
-// Deals a launch out: wide tiles of `pixels` a thread first, then `narrow` tiles of 32 pixels a scheduler (and what is left of
-// the rows' groups), which even out the end.  With `rounds` or fewer tiles a warp the launch does without a queue.  Returns the
-// grid: the shared tables allow one CTA per SM.
-static unsigned deal_exact(LambdaArgs* a, int pixels, int narrow, int rounds, int sm_count) {
-    const long long wide_px = a->n_pixels - narrow * 32LL * 4 * sm_count;
+// Deals a launch out: `wide_tiles` of `pixels` a thread first (as far as the rows' whole groups hold them), then tiles of 32
+// pixels, which even out the end.  With `rounds` or fewer tiles a warp the launch does without a queue.  Returns the grid: the
+// shared tables allow one CTA per SM.
+static unsigned deal_exact(LambdaArgs* a, int pixels, long long wide_tiles, int rounds, int sm_count) {
     const long long groups = a->n_pixels / a->width / pixels * a->width / 32;   // wide tiles in the rows' whole groups
-    a->wide_tiles = std::max(0LL, std::min(wide_px / (32 * pixels), groups));
+    a->wide_tiles = std::max(0LL, std::min(wide_tiles, groups));
     const long long warp_tiles = a->wide_tiles + (a->n_pixels - a->wide_tiles * 32 * pixels + 31) / 32;
     if (warp_tiles <= (long long)rounds * kExactThreads / 32 * sm_count) a->queue = nullptr;
     return (unsigned)std::min<long long>(warp_tiles, sm_count);
@@ -66,16 +66,14 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
                                 int sm_count, cudaStream_t st) {
     if (args.n_pixels <= 0) return cudaSuccess;
     LambdaArgs a = args;
-    // a periodic sequence can run an instance of this kernel made for its patterns
+    // A periodic sequence can run an instance of this kernel made for its patterns.
     // Frames of up to 40 tiles of 32 a scheduler go in such tiles alone: with 4 / 8 / 16 / 32 / all of them 800 x 800 of "AB"
     // 100 + 1000 over [0.01,3.99]^2 takes 471 / 471 / 471 / 447 / 426 us and 512 x 512 over [2,4]^2 215 / 210 / 202 / 202 / 202;
-    // 1920 x 1080 of "ABC" 300 + 3000 3675 / 3694 / 3701 / 3717 / 3758.  The generic kernel's choice of a body serves all of a
-    // thread's pixels (1277 x 719 of 37 letters 864 / 892 / 930 / 989 / 1028), but fewer than six tiles a scheduler are better
-    // all small: 190 x 223 of "AABAB" 27 + 270 45 us, with some wide ones 73.
+    // 1920 x 1080 of "ABC" 300 + 3000 3675 / 3694 / 3701 / 3717 / 3758.
     // Orbits of one length end on an SM's 16 warps at once, which then take 16 tiles from the queue where others get none: two
     // rounds of tiles and fewer are dealt out beforehand (315 x 305 of "AB" 82 + 821 over [3.4,4]x[2.5,3.4]: 126 -> 104 us).
-    const int small = 40;
-    unsigned grid = deal_exact(&a, kExactPixels, a.n_pixels <= small * 32LL * 4 * sm_count ? small : 8, 2, sm_count);
+    const long long schedulers = 4LL * sm_count, tiles = (a.n_pixels + 31) / 32;
+    unsigned grid = deal_exact(&a, kExactPixels, tiles <= 40 * schedulers ? 0 : (tiles - 8 * schedulers) / kExactPixels, 2, sm_count);
     bool launched = false;
     const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads, kExactSmemBytes,
                                              spec_mode(), &launched);
@@ -83,10 +81,29 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     bool has_c = false;
     const int words = a.acc_word0 + (a.iterations > 0 ? min(a.acc_wrap, (a.iterations - 1) / kStepsPerWord + 1) : 0);
     for (int i = 0; i < words; ++i) has_c = has_c || (a.sel[i] & 0xAAAAAAAAu);
+    // The generic kernel's choice of a body serves all of a thread's pixels, so that its large frames have four small tiles a
+    // scheduler only (1277 x 719 of 37 letters with 4 / 8 / 16 / 32 / all 864 / 892 / 930 / 989 / 1028 us).  Frames of few tiles go
+    // in small ones alone, through a kernel that has four steps to a body; more, up to what one round of warps holds, in as few
+    // wide tiles as fill it.  Runs too short for cycles make even tiles: there a round begins earlier (454 x 247 of 37 letters 24 + 218
+    // 56 us in small tiles, 49 in a round), and a few rounds are dealt out beforehand (685 x 485, 11 + 111: 65 us from the queue, 60).
+    // 37 letters in four small tiles a scheduler beyond the wide ones, and small ones alone up to six / this: 64 x 32 100 + 4000 296 /
+    // 249 us, 437 x 385 230 + 2304 over [3.9,4]^2 552 / 457, 357 x 213 of "ABBAB" 24 + 1700 over [0,4]^2 219 / 194.
+    const bool uneven = a.acc_period && a.iterations >= a.acc_chunk + kLeastLeft;
     a.queue = args.queue;
-    grid = deal_exact(&a, kGenericPixels, a.n_pixels <= 6 * 32LL * 4 * sm_count ? 6 : 4, 1, sm_count);
-    return has_c ? launch_exact_generic<true>(a, out64, out32, steps, grid, st)
-                 : launch_exact_generic<false>(a, out64, out32, steps, grid, st);
+    if (tiles <= (uneven ? 6 : 5) * schedulers) {
+        grid = deal_exact(&a, 1, 0, 1, sm_count);
+        return has_c ? launch_exact_generic<1, true, 2>(a, out64, out32, steps, grid, st)
+                     : launch_exact_generic<1, false, 4>(a, out64, out32, steps, grid, st);
+    }
+    long long wide = (tiles - 4 * schedulers) / kGenericPixels;
+    if (tiles <= 4 * kGenericPixels * schedulers) wide = (tiles - 2 * schedulers - 1) / (2 * schedulers) * schedulers;
+    else if (!uneven && tiles <= 8 * kGenericPixels * schedulers) {
+        wide = (tiles - 2 * schedulers) / (kGenericPixels * schedulers) * schedulers;
+        a.queue = nullptr;
+    }
+    grid = deal_exact(&a, kGenericPixels, wide, 1, sm_count);
+    return has_c ? launch_exact_generic<kGenericPixels, true, 2>(a, out64, out32, steps, grid, st)
+                 : launch_exact_generic<kGenericPixels, false, 2>(a, out64, out32, steps, grid, st);
 }
 
 // ---------------------------------------------------------------------------------------------

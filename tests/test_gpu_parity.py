@@ -162,6 +162,21 @@ def test_every_tile_of_a_launch_is_walked_once(engine, port, kernel_path, path, 
     assert np.array_equal(r["lambda32"].view(np.uint32), lam.astype(np.float32).view(np.uint32))
 
 
+# The generic kernel's ways of dealing a frame out change at 5 or 6, 12 and 24 tiles of 32 pixels a scheduler (592 of them).
+@pytest.mark.parametrize("rows,iterations,small", [(40, 90, True), (41, 90, False), (48, 300, True), (49, 300, False), (96, 300, False),
+                                                   (97, 300, False), (96, 90, False), (97, 90, False), (192, 90, False), (193, 90, False)])
+@pytest.mark.parametrize("c", [None, 3.6], ids=["AB", "ABC"])
+def test_generic_frames_at_the_edges_of_their_deals(engine, port, kernel_path, rows, iterations, small, c):
+    """The lambda bits and the steps of every way, and that frames of few tiles take the kernel of one pixel a thread."""
+    kernel_path("generic")
+    kw = dict(min_x=2.4, max_x=4.05, min_y=2.2, max_y=4.02, width=2368, height=rows, iterations=iterations, warmup=21, c=c,
+              sequence="ABBABAABBBABAABABBBAABABAABBBABBAAABA" if c is None else "ABCABBAABCACBBABAABABC")
+    r = engine.render(L.make_params(**kw), want=("lambda",))
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps
+    assert ("k_lambda_exact<1," in engine.lib.lyap_last_kernel().decode()) == small
+
+
 @pytest.mark.parametrize("kw", [
     dict(sequence="AB", max_x=1.1, max_y=1.1), dict(sequence="BBBBBBAAAAAA", max_x=4.0, max_y=0.3),
     dict(sequence="ABB" * 15 + "A", max_x=300.0, max_y=0.01),                           # some parameters above the rule's 256
