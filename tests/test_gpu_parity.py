@@ -263,8 +263,8 @@ def test_seeded_random_cases_against_the_oracle(engine, port, kernel_path):
 CYCLE_CASES = [
     # window, size, sequence, iterations, warm-up, c: what is at its edge
     ((2.0, 3.9, 2.0, 3.9), (129, 61), "AB", 1000, 100, None),        # (2, 2): x = 1/2 for good, no term at all
-    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 79, 0, None),    # one step too few are left behind the ninth chunk
-    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 80, 0, None),    # just enough
+    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 79, 0, None),    # whole chunks and a rest, no warm-up
+    ((2.0, 2.4, 3.0, 4.0), (64, 48), "AB", 32 * 9 + 80, 0, None),
     ((2.5, 4.0, 2.5, 4.0), (131, 67), "AABAB", 2011, 200, None),     # whole and single steps behind the last chunk
     ((3.4, 4.0, 2.5, 3.4), (97, 50), "BBBBBBAAAAAA", 4000, 500, None),
     ((3.815, 3.825, 3.445, 3.455), (95, 40), "ABC", 3000, 300, 3.7),
@@ -296,3 +296,26 @@ def test_orbits_that_come_into_cycles(engine, port, monkeypatch, case, generic):
     assert 0 <= taken < steps
     if len(sequence) < 80 and iterations > 1000 and not (generic and sequence == "A"):   # no chunk holds nine, and there is no reference value
         assert taken > 0
+
+
+@pytest.mark.parametrize("sequence,chunk,iterations,left", [
+    ("AB", 48, 255, 0), ("AB", 48, 256, 160),                       # one step too few behind the second chunk, and just enough
+    ("AABAB", None, 1000, None),                                    # whatever the chunk
+    ("AB" * 39 + "BA", 80, 319, 0), ("AB" * 39 + "BA", 80, 320, 160), ("AB" * 39 + "BA", 80, 2003, 1843),
+    ("AB" * 39 + "BAB", None, 2003, 0),                             # a period of 81 is not looked for
+], ids=lambda v: str(len(v)) if isinstance(v, str) else str(v))
+@pytest.mark.parametrize("path", ["prebuilt", "generic"])
+def test_where_walking_stops_in_a_cycle(engine, port, kernel_path, path, sequence, chunk, iterations, left):
+    """A window in which every orbit reaches its cycle within the first chunk, so that all are found in it behind the second and
+    leave the steps from there on, if they are 160 at least: the bits, and exactly that many steps taken from cycles."""
+    kernel_path(path)
+    kw = dict(min_x=2.05, max_x=2.15, min_y=2.05, max_y=2.15, width=37, height=43, sequence=sequence, iterations=iterations, warmup=0)
+    before = engine.cycle_steps()
+    r = engine.render(L.make_params(**kw), want=("lambda",))
+    taken = engine.cycle_steps() - before
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps == 37 * 43 * iterations
+    if left is None:
+        assert 37 * 43 * (iterations - 2 * 80) <= taken <= 37 * 43 * iterations
+    else:
+        assert taken == 37 * 43 * left and (chunk is None or left in (0, iterations - 2 * chunk))
