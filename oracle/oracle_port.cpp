@@ -14,7 +14,7 @@
 //   oracle_colorize         web/fractal_renderer.js:177-198  renderFractal up to the ImageData store
 //   oracle_glow             web/fractal_renderer.js:313-334  applyGlow (browser-defined; this project's reading)
 // and, of the engine's own fast modes, which the reference has no counterpart of:
-//   oracle_fused_lambda     the fused step in float or double, its logarithms summed in extended precision
+//   oracle_fused_lambda     the fused step in float or double, or the reference's step, its logarithms summed in extended precision
 //
 // Differences from the reference, on purpose:
 //   * rows are addressed by their GLOBAL index (r_y = min_y + dy*y_global with the global dy), so
@@ -131,8 +131,9 @@ uint64_t oracle_lambda_rows(double min_x, double max_x, double min_y, double max
 }   // extern "C"
 
 // One pixel of a fused mode: t = r*x, derivative |fma(-2,t,r)|, x' = fma(-t,x,t), in T; the reference's rules for terms
-// and exits.  The engine multiplies the derivatives where this sums their logarithms.
-template <typename T>
+// and exits.  SAME_ORBIT: the reference's own step, x' = (r*x)*(1-x), and the derivative as the product of r and |1 - 2x|, unrounded.
+// The engine multiplies the derivatives where this sums their logarithms.
+template <typename T, bool SAME_ORBIT = false>
 static double fused_pixel(double r_x, double r_y, double r_c, const uint8_t* sel, int seq_len, int warmup, int iterations,
                           uint64_t* steps) {
     if (r_x <= 0.0 || r_y <= 0.0) return -5.0;
@@ -143,13 +144,13 @@ static double fused_pixel(double r_x, double r_y, double r_c, const uint8_t* sel
     for (int64_t i = 0; i < (int64_t)warmup + iterations; ++i) {
         const T rr = r[sel[i % seq_len]], t = rr * x;
         if (i >= warmup) {
-            const T d = std::fabs(std::fma((T)-2, t, rr));
-            if (d > (T)0) {
-                sum += std::log((long double)d);
+            const long double d = SAME_ORBIT ? (long double)rr * std::fabs(std::fma((T)-2, x, (T)1)) : (long double)std::fabs(std::fma((T)-2, t, rr));
+            if (d > 0.0L) {
+                sum += std::log(d);
                 ++terms;
             }
         }
-        x = std::fma(-t, x, t);
+        x = SAME_ORBIT ? t * ((T)1 - x) : std::fma(-t, x, t);
         ++*steps;
         if (!(x > (T)0 && x < (T)1)) break;
     }
@@ -159,7 +160,7 @@ static double fused_pixel(double r_x, double r_y, double r_c, const uint8_t* sel
 extern "C" {
 
 uint64_t oracle_fused_lambda(double min_x, double max_x, double min_y, double max_y, int width, int height, const char* sequence,
-                             int seq_len, int iterations, int warmup, int c_enabled, double c_value, int single, double* out) {
+                             int seq_len, int iterations, int warmup, int c_enabled, double c_value, int flavour, double* out) {   // 0 fused double, 1 fused float, 2 the reference's orbit
     const double dx = (max_x - min_x) / (width - 1.0), dy = (max_y - min_y) / (height - 1.0);
     std::vector<uint8_t> sel(seq_len);
     for (int j = 0; j < seq_len; ++j) sel[j] = sequence[j] == 'A' ? 0 : (sequence[j] == 'C' && c_enabled ? 2 : 1);
@@ -168,9 +169,8 @@ uint64_t oracle_fused_lambda(double min_x, double max_x, double min_y, double ma
     for (int y = 0; y < height; ++y) {
         uint64_t steps = 0;
         for (int x = 0; x < width; ++x)
-            out[(int64_t)y * width + x] =
-                single ? fused_pixel<float>(min_x + dx * x, min_y + dy * y, c_value, sel.data(), seq_len, warmup, iterations, &steps)
-                       : fused_pixel<double>(min_x + dx * x, min_y + dy * y, c_value, sel.data(), seq_len, warmup, iterations, &steps);
+            out[(int64_t)y * width + x] = (flavour == 2 ? fused_pixel<double, true> : flavour == 1 ? fused_pixel<float> : fused_pixel<double>)(
+                min_x + dx * x, min_y + dy * y, c_value, sel.data(), seq_len, warmup, iterations, &steps);
         total += steps;
     }
     return total;

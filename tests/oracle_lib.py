@@ -67,12 +67,13 @@ class Port:
                                             row_stride, _dp(out))
         return out, int(steps)
 
-    def fused_lambda(self, min_x, max_x, min_y, max_y, width, height, sequence, iterations, warmup, c=None, single=False):
-        """The whole frame in the fused fp64 (single: fp32) step, logarithms summed in extended precision -> (array, steps)."""
+    def fused_lambda(self, min_x, max_x, min_y, max_y, width, height, sequence, iterations, warmup, c=None, single=False, same_orbit=False):
+        """The whole frame in the fused fp64 (single: fp32; same_orbit: the reference's) step, logarithms summed in extended
+        precision -> (array, steps)."""
         out = np.empty((height, width), dtype=np.float64)
         seq = sequence.encode("latin-1")
         steps = self.lib.oracle_fused_lambda(min_x, max_x, min_y, max_y, width, height, seq, len(seq), iterations, warmup,
-                                             0 if c is None else 1, 0.0 if c is None else c, 1 if single else 0, _dp(out))
+                                             0 if c is None else 1, 0.0 if c is None else c, 2 if same_orbit else 1 if single else 0, _dp(out))
         return out, int(steps)
 
     def minmax(self, v):

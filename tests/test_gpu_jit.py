@@ -105,7 +105,7 @@ def test_specialised_fast_kernels_agree_with_the_precompiled_ones(engine, kernel
     """Fast modes: moving the exponent out of the running product is exact, so where the products are stripped does
     not change their value: pixels whose run was regular get the precompiled kernel's bits.  Pixels that had a chunk
     redone step by step (an exit, a zero derivative) may differ in the last digits, because the two kernels cut the
-    run into chunks at different steps and a redone chunk adds logs one by one instead of multiplying."""
+    run into chunks at different steps and a redone chunk's derivatives are multiplied up in doubles, apart from the running product."""
     tol = 2e-4 if mode == L.MODE_FAST_FP32 else 1e-10
     for case in CASES[:6]:
         kw = dict(min_x=2.3, max_x=4.1, min_y=2.2, max_y=4.05, width=257, height=45, mode=mode, **case)
@@ -247,16 +247,18 @@ def test_fast_modes_on_falls_that_a_large_or_undefined_parameter_ends(engine, po
 def test_fast_modes_on_orbits_that_come_into_cycles(engine, port, kernel_path, path, size):
     """Turns of a cycle added up instead of walked, on both cuts of a frame into threads' pixels: the exits and the count of
     steps are the restatement's, and lambda differs from its extended sum by the rounding of a factor a step (2^-24 or 2^-53 of
-    it, / ln 2 in the mean) and of a few operations at the end."""
+    it, / ln 2 in the mean) and of a few operations at the end; on the reference's orbit also of the parameters' logarithms, of
+    which there are as many as steps, each below log2(4)."""
     kernel_path(path)
     for sequence, iterations in (("AAB", 1000), ("AAB", 72 * 9), ("AB", 96 * 8 + 95), ("AB" * 18 + "A", 1500)):
         kw = dict(min_x=2.1, max_x=3.0, min_y=2.2, max_y=3.4, width=size[0], height=size[1], sequence=sequence, iterations=iterations,
                   warmup=33)
-        for mode, unit in ((L.MODE_FAST_FP64, 2.0 ** -53), (L.MODE_FAST_FP32, 2.0 ** -24)):
-            want, steps = port.fused_lambda(**kw, single=mode == L.MODE_FAST_FP32)
+        for mode, unit in ((L.MODE_FAST_FP64, 2.0 ** -53), (L.MODE_FAST_FP32, 2.0 ** -24), (L.MODE_FAST_FP64_ORBIT, 2.0 ** -53)):
+            want, steps = port.fused_lambda(**kw, single=mode == L.MODE_FAST_FP32, same_orbit=mode == L.MODE_FAST_FP64_ORBIT)
             before = engine.cycle_steps()
             r = engine.render(L.make_params(**kw, mode=mode), want=("lambda",))
             assert r["stats"].executed_steps == steps
-            bound = 1.001 * unit / np.log(2.0) + 8 * 2.0 ** -53 * np.max(np.abs(want))
+            ends = np.max(np.abs(want)) + (2.0 if mode == L.MODE_FAST_FP64_ORBIT else 0.0)
+            bound = 1.001 * unit / np.log(2.0) + 8 * 2.0 ** -53 * ends
             assert np.max(np.abs(r["lambda"] - want)) < bound, (sequence, iterations, mode)
             assert size != (64, 47) or engine.cycle_steps() > before   # in the smaller frames a slow orbit holds every tile up
