@@ -15,16 +15,17 @@ def test_specialised_kernel_source_compiles_for_sm_100a():
         from cuda.bindings import nvrtc
     except ImportError:
         nvrtc = pytest.importorskip("cuda.nvrtc")
+    from lyapunovfractalwasm_b200 import build
     read = lambda n: open(os.path.join(CSRC, n)).read().encode()
     names = [b"lyap_exact_kernel.cuh", b"lyap_kernels_fast.cuh", b"lyap_args.h", b"lyap_math.h", b"lyap_tables.h"]
     main = b'#include "lyap_exact_kernel.cuh"\n#include "lyap_kernels_fast.cuh"\n'
     # "AABAB": group patterns AA BA BA AB AB for both regions (warm-up 200 is a whole number of periods)
     common = [b"--gpu-architecture=sm_100a", b"--fmad=false", b"--std=c++17", b"-DLYAP_SPEC_KG=5",
               b"-DLYAP_SPEC_WU_PATS=0x44110ull", b"-DLYAP_SPEC_ACC_PATS=0x44110ull"]
-    for symbol, kind in ((b"k_lambda_exact_spec", [b"-DLYAP_SPEC_EXACT=1", b"-DLYAP_SPEC_THREADS=512", b"-DLYAP_SPEC_P=3"]),
-                         (b"k_lambda_fast_spec", [b"-DLYAP_SPEC_FAST=FusedF64", b"-DLYAP_SPEC_THREADS=512", b"-DLYAP_SPEC_P=4"]),
-                         (b"k_lambda_fast_spec", [b"-DLYAP_SPEC_FAST=FusedF32", b"-DLYAP_SPEC_THREADS=512", b"-DLYAP_SPEC_P=2"]),
-                         (b"k_lambda_fast_spec", [b"-DLYAP_SPEC_FAST=OrbitF64", b"-DLYAP_SPEC_THREADS=512", b"-DLYAP_SPEC_P=4"])):
+    kinds = [b"-DLYAP_SPEC_EXACT=1", b"-DLYAP_SPEC_FAST=FusedF64", b"-DLYAP_SPEC_FAST=FusedF32", b"-DLYAP_SPEC_FAST=OrbitF64"]
+    for which, pixels, threads in build.PREBUILT_SHAPES:   # the shapes the launchers ask for
+        symbol = b"k_lambda_exact_spec" if which == 0 else b"k_lambda_fast_spec"
+        kind = [kinds[which], b"-DLYAP_SPEC_THREADS=%d" % threads, b"-DLYAP_SPEC_P=%d" % pixels]
         err, prog = nvrtc.nvrtcCreateProgram(main, b"spec.cu", len(names), [read(n.decode()) for n in names], names)
         assert err == nvrtc.nvrtcResult.NVRTC_SUCCESS
         opts = common + kind
