@@ -499,12 +499,22 @@ def test_a_captured_lambda_launch_shares_nothing_with_direct_ones(engine):
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=mine, capture_error_mode="relaxed"):
             engine.lambda_device(p, d_lambda=captured.data_ptr())
-        for _ in range(4):
+        engine.sync()
+        taken = engine.cycle_steps()
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert engine.cycle_steps() == taken   # a captured launch holds nothing of the context's
+        for _ in range(24):
+            captured.fill_(float("nan"))
+            direct.fill_(float("nan"))
+            torch.cuda.synchronize()
             with torch.cuda.stream(other):
                 graph.replay()
             engine.lambda_device(p, d_lambda=direct.data_ptr())
-        torch.cuda.synchronize()
+            torch.cuda.synchronize()
+            for got in (captured, direct):
+                assert np.array_equal(got.cpu().numpy().view(np.uint64), want.ravel().view(np.uint64))
+        assert engine.cycle_steps() > taken
     finally:
         engine.set_stream(None)
-    for got in (captured, direct):
-        assert np.array_equal(got.cpu().numpy().view(np.uint64), want.ravel().view(np.uint64))
