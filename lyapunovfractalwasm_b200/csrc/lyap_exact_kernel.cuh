@@ -441,13 +441,13 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         in_cycle[p] = false;
         no_cycle[p] = careful_only[p];
     }
-    // Behind every whole chunk of the accumulation, whose steps are a multiple of the period: the pixels whose orbit stands
-    // where it stood a chunk ago or at the reference value are in a cycle, and when all of the warp's are (or have ended), the
-    // `left` steps from `next` on are added up from one turn of each (cycle_steps).  Lanes that are in one before the others
-    // go on walking -- refilling them with other pixels costs more in warm-ups run for a part of a warp than it saves --, but
-    // for those in `redone`, which had this chunk walked step by step (a derivative of zero) and would have every other.  The
-    // generic kernel has no registers left for the reference value (it spills: 1.02 -> 1.07 ms); its chunks hold cycles of
-    // three where they can.
+    // Behind every whole chunk of the accumulation, whose steps are a multiple of the period, while steps enough are left for it
+    // to pay: the pixels whose orbit stands where it stood a chunk ago or at the reference value are in a cycle, and when all of
+    // the warp's are (or have ended), the `left` steps from `next` on are added up from one turn of each (cycle_steps).  Lanes
+    // that are in one before the others go on walking -- refilling them with other pixels costs more in warm-ups run for a part
+    // of a warp than it saves --, but for those in `redone`, which had this chunk walked step by step (a derivative of zero) and
+    // would have every other.  The generic kernel has no registers left for the reference value (it spills: 1.02 -> 1.07 ms); its
+    // chunks hold cycles of three where they can.
     auto cycles = [&](const double (&sx)[P], unsigned redone, const unsigned* sel, int wrap, int period, int next, int left) {
         bool all = true;
 #pragma unroll
@@ -461,7 +461,6 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
 #pragma unroll
             for (int p = 0; p < P; ++p) ref[p] = x[p];
         }
-        if (left < kLeastLeft) return;
         const bool every = __all_sync(0xFFFFFFFFu, all);
         if (!every && !__any_sync(0xFFFFFFFFu, redone != 0)) return;
 #pragma unroll
@@ -557,7 +556,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
                         }
                     }
                 }
-                if (acc && n == CS) cycles(sx, redone, sel, wrap, BS, s + n, nsteps - s - n);
+                if (acc && n == CS && left >= CS + kLeastLeft) cycles(sx, redone, sel, wrap, BS, s + n, left - n);
                 s += n;
             }
             continue;
@@ -613,7 +612,8 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
                     }
                 }
             }
-            if (acc && a.acc_period && n == chunk) cycles(sx, redone, sel, wrap, a.acc_period, s + n, nsteps - s - n);
+            const int left = nsteps - s - n;
+            if (acc && a.acc_period && left >= kLeastLeft) cycles(sx, redone, sel, wrap, a.acc_period, s + n, left);
             s += n;
         }
     }

@@ -72,8 +72,16 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     // 1920 x 1080 of "ABC" 300 + 3000 3675 / 3694 / 3701 / 3717 / 3758.
     // Orbits of one length end on an SM's 16 warps at once, which then take 16 tiles from the queue where others get none: two
     // rounds of tiles and fewer are dealt out beforehand (315 x 305 of "AB" 82 + 821 over [3.4,4]x[2.5,3.4]: 126 -> 104 us).
+    // Runs long enough for cycles to be cut short make uneven tiles, which small ones and the queue even out.  Those of shorter runs
+    // end together: whole rounds of wide tiles over the schedulers, all dealt out beforehand (744 x 659 of "ABC" 24 + 213 137 -> 122 us,
+    // 1074 x 549 of "AABAB" 25 + 158 132 -> 118; 550 x 530 of "BBBBBBAAAAAA" 20 + 399 over [2,4]^2 is better in small ones, 126 us
+    // against 166).
     const long long schedulers = 4LL * sm_count, tiles = (a.n_pixels + 31) / 32;
-    unsigned grid = deal_exact(&a, kExactPixels, tiles <= 40 * schedulers ? 0 : (tiles - 8 * schedulers) / kExactPixels, 2, sm_count);
+    const bool uneven = a.acc_period && a.iterations >= 300;
+    long long wide = (tiles - 2 * schedulers) / (kExactPixels * schedulers) * schedulers;
+    if (uneven) wide = tiles <= 40 * schedulers ? 0 : (tiles - 8 * schedulers) / kExactPixels;
+    else a.queue = nullptr;
+    unsigned grid = deal_exact(&a, kExactPixels, wide, 2, sm_count);
     bool launched = false;
     const cudaError_t e = launch_lambda_spec(a, out64, out32, steps, grid, st, 0, kExactPixels, kExactThreads, kExactSmemBytes,
                                              spec_mode(), &launched);
@@ -84,18 +92,17 @@ cudaError_t launch_lambda_exact(const LambdaArgs& args, double* out64, float* ou
     // The generic kernel's choice of a body serves all of a thread's pixels, so that its large frames have four small tiles a
     // scheduler only (1277 x 719 of 37 letters with 4 / 8 / 16 / 32 / all 864 / 892 / 930 / 989 / 1028 us).  Frames of few tiles go
     // in small ones alone, through a kernel that has four steps to a body; more, up to what one round of warps holds, in as few
-    // wide tiles as fill it.  Runs too short for cycles make even tiles: there a round begins earlier (454 x 247 of 37 letters 24 + 218
-    // 56 us in small tiles, 49 in a round), and a few rounds are dealt out beforehand (685 x 485, 11 + 111: 65 us from the queue, 60).
+    // wide tiles as fill it.  Short runs' even tiles: there a round begins earlier (454 x 247 of 37 letters 24 + 218 56 us in small
+    // tiles, 49 in a round), and a few rounds are dealt out beforehand (685 x 485, 11 + 111: 65 us from the queue, 60).
     // 37 letters in four small tiles a scheduler beyond the wide ones, and small ones alone up to six / this: 64 x 32 100 + 4000 296 /
     // 249 us, 437 x 385 230 + 2304 over [3.9,4]^2 552 / 457, 357 x 213 of "ABBAB" 24 + 1700 over [0,4]^2 219 / 194.
-    const bool uneven = a.acc_period && a.iterations >= a.acc_chunk + kLeastLeft;
     a.queue = args.queue;
     if (tiles <= (uneven ? 6 : 5) * schedulers) {
         grid = deal_exact(&a, 1, 0, 1, sm_count);
         return has_c ? launch_exact_generic<1, true, 2>(a, out64, out32, steps, grid, st)
                      : launch_exact_generic<1, false, 4>(a, out64, out32, steps, grid, st);
     }
-    long long wide = (tiles - 4 * schedulers) / kGenericPixels;
+    wide = (tiles - 4 * schedulers) / kGenericPixels;
     if (tiles <= 4 * kGenericPixels * schedulers) wide = (tiles - 2 * schedulers - 1) / (2 * schedulers) * schedulers;
     else if (!uneven && tiles <= 8 * kGenericPixels * schedulers) {
         wide = (tiles - 2 * schedulers) / (kGenericPixels * schedulers) * schedulers;

@@ -177,6 +177,17 @@ def test_generic_frames_at_the_edges_of_their_deals(engine, port, kernel_path, r
     assert ("k_lambda_exact<1," in engine.lib.lyap_last_kernel().decode()) == small
 
 
+# Short runs of an instance go in whole rounds of wide tiles from 4 small ones a scheduler on, long ones from 40 on.
+@pytest.mark.parametrize("rows,iterations", [(31, 90), (32, 90), (48, 90), (49, 299), (320, 300), (321, 300)])
+def test_instances_at_the_edges_of_their_deals(engine, port, kernel_path, rows, iterations):
+    kernel_path("prebuilt")
+    kw = dict(min_x=2.4, max_x=4.05, min_y=2.2, max_y=4.02, width=2368, height=rows, sequence="AABAB", iterations=iterations, warmup=25)
+    r = engine.render(L.make_params(**kw), want=("lambda",))
+    lam, steps = oracle_rows(port, kw)
+    assert same_bits(r["lambda"], lam) and r["stats"].executed_steps == steps
+    assert "built for the patterns" in engine.lib.lyap_last_kernel().decode()
+
+
 @pytest.mark.parametrize("kw", [
     dict(sequence="AB", max_x=1.1, max_y=1.1), dict(sequence="BBBBBBAAAAAA", max_x=4.0, max_y=0.3),
     dict(sequence="ABB" * 15 + "A", max_x=300.0, max_y=0.01),                           # some parameters above the rule's 256
