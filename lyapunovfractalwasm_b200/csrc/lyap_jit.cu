@@ -12,7 +12,11 @@
 #include <dlfcn.h>
 #include <nvrtc.h>
 
+#include <unistd.h>
+
 #include <algorithm>
+#include <chrono>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -165,6 +169,32 @@ bool compile_cubin(const Key& key, std::vector<char>* out, std::string* note) {
     n.cubin(prog, cubin.data());
     n.destroy(&prog);
     return true;
+}
+
+// Background compilations that run now, and a process that ends waits for: NVRTC's own static objects must not be destroyed under
+// one.  Handlers of exit() run last registered first, and NVRTC registers some of its own while it compiles for the first time, so
+// the waiting one is registered behind a first compilation of next to nothing (0.05 s, on the background thread).
+std::condition_variable& g_idle = *new std::condition_variable;
+int g_running = 0;
+pid_t g_pid = 0;   // a forked child has none of the threads
+
+void wait_for_background() {
+    std::unique_lock<std::mutex> lk(g_mu);
+    if (getpid() == g_pid) g_idle.wait_for(lk, std::chrono::seconds(30), [] { return g_running == 0; });
+}
+
+void wait_at_exit() {
+    static std::once_flag& once = *new std::once_flag;
+    std::call_once(once, [] {
+        Nvrtc& n = nvrtc();
+        nvrtcProgram prog = nullptr;
+        static const char* const opts[] = {"--gpu-architecture=sm_100a"};
+        if (n.ok && n.create(&prog, "__global__ void nothing(float* p) { p[threadIdx.x] *= 2.0f; }", "first.cu", 0, nullptr, nullptr) == NVRTC_SUCCESS) {
+            n.compile(prog, 1, opts);
+            n.destroy(&prog);
+        }
+        std::atexit(wait_for_background);
+    });
 }
 
 // Loads the (cached) cubin into the current device's context and looks the kernel up.
@@ -327,11 +357,15 @@ cudaError_t launch_lambda_spec(const LambdaArgs& a, double* out64, float* out32,
                     e.failed = true;
                 } else if (state == 0) {
                     state = 1;
+                    ++g_running;
+                    g_pid = getpid();
                     std::thread([key, ck]() {
                         std::vector<char> cubin;
                         std::string note;
+                        wait_at_exit();
                         const bool ok = compile_cubin(key, &cubin, &note);
                         std::lock_guard<std::mutex> lk2(g_mu);
+                        if (--g_running == 0) g_idle.notify_all();
                         if (ok) {
                             g_cubins[ck] = std::move(cubin);
                             g_background[ck] = 0;
