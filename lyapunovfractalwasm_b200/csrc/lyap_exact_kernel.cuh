@@ -385,14 +385,18 @@ __device__ __forceinline__ void fast_chunk(double (&x)[P], double (&lyap)[P], do
     constexpr int U = HAS_C ? 2 : UNROLL;
     unsigned pat = HAS_C ? word : compress_even_bits(word);
     constexpr int kBits = HAS_C ? 2 * U : U;
-    int left = n;
+    const int groups = n / U;
 #pragma unroll 1
-    for (; left >= U; left -= U) {
+    for (int h = 0; h < groups; ++h) {
         dispatch_group<P, ACC, HAS_C, U>(x, lyap, rA, rB, rC, pat & ((1u << kBits) - 1u), lane_off);
         pat >>= kBits;
     }
+    if constexpr (U == 2) {
+        if (n % U) fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word >> (2 * (n - 1)), lane_off);
+    } else {
 #pragma unroll 1
-    for (; left > 0; --left) fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word >> (2 * (n - left)), lane_off);
+        for (int j = n & ~(U - 1); j < n; ++j) fast_group<P, ACC, HAS_C, 1>(x, lyap, rA, rB, rC, word >> (2 * j), lane_off);
+    }
 }
 
 // ---- run-time specialisation -------------------------------------------------------------------
@@ -565,7 +569,7 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
         static_assert(2 * kStepsPerWord <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
         const unsigned* sel = a.sel + word0;
         const int chunk = acc ? a.acc_chunk : 2 * kStepsPerWord;
-        int s = 0, wi = 0;
+        int s = 0, wi = 0, in_word = 0;   // step s is step in_word of word wi
         while (s < nsteps) {
             bool all_done = true;
 #pragma unroll
@@ -573,7 +577,10 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             if (__all_sync(0xFFFFFFFFu, all_done)) break;
 
             const int n = min(chunk, nsteps - s);
-            if (acc && a.acc_period) wi = 0;   // whole periods lie behind: this chunk has the selectors of the first
+            // Whole periods lie behind this chunk, it has the selectors of the first: read from its words' beginnings (37 letters
+            // 1277 x 719 849 -> 832 us).  With three parameters that makes slower code of the whole loop (1783 x 1722 of "ABC"
+            // 172 + 1719, nearly all in cycles, 2.57 -> 2.77 ms), and the words go on through the chunks.
+            if (!HAS_C && acc && a.acc_period) wi = 0;
             double sx[P], sl[P];
 #pragma unroll
             for (int p = 0; p < P; ++p) {
@@ -583,8 +590,13 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
 #pragma unroll 1
             for (int k = 0; k < n; k += kStepsPerWord) {
                 const int m = min(kStepsPerWord, n - k);
-                const unsigned word = sel[wi];
-                if (++wi == wrap) wi = 0;
+                const int after = wi + 1 == wrap ? 0 : wi + 1;
+                const unsigned word = HAS_C ? __funnelshift_r(sel[wi], sel[after], 2 * in_word) : sel[wi];
+                in_word += m;
+                if (!HAS_C || in_word >= kStepsPerWord) {
+                    in_word -= kStepsPerWord;
+                    wi = after;
+                }
                 if (acc) fast_chunk<P, true, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
                 else fast_chunk<P, false, HAS_C, UNROLL>(x, lyap, rA, rB, rC, word, m, lane_off);
             }
