@@ -494,6 +494,10 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
     // after which its orbit stood where it had stood a chunk before
     constexpr int kWalks = -1, kCareful = -2, kDone = -3;
     int state[P];
+    // a thread's own places for its sums then: registers for them would be taken from the loop (4096^2 of "AABAB" 200 + 2000
+    // in fp32 3.27 -> 3.20 ms)
+    __shared__ T kept_prod[P][THREADS];
+    __shared__ int kept_esum[P][THREADS];
     // pixel p's place in the launch, or -1 where there is none
     auto place = [&](int p) -> long long {
         const long long group = at / a.width;
@@ -621,11 +625,7 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
 #pragma unroll
             for (int p = 0; p < P; ++p) {
                 if (state[p] == kDone) continue;
-                if (state[p] >= 0) {   // sums stay as they were when it turned; x comes back by itself
-                    prod[p] = sp[p];
-                    esum[p] = se[p];
-                    continue;
-                }
+                if (state[p] >= 0) continue;   // its sums are kept (and run on unused), x comes back by itself
                 // a zero derivative (or a product that underflowed) shows as exponent field 0
                 const bool regular = state[p] == kWalks && (kSign * x[p] > (T)0 && kSign * x[p] < (T)1) && (!acc || emin[p] != 0);
                 if (regular) {
@@ -637,7 +637,11 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                             nuse[p][1] += cuse[1];
                             nuse[p][2] += cuse[2];
                         }
-                        if (s < whole - kLeastChunks * chunk && x[p] == sx[p]) state[p] = s + n;
+                        if (s < whole - kLeastChunks * chunk && x[p] == sx[p]) {
+                            state[p] = s + n;
+                            kept_prod[p][threadIdx.x] = prod[p];
+                            kept_esum[p][threadIdx.x] = esum[p];
+                        }
                     }
                     my_steps += n;
                 } else {
@@ -659,11 +663,11 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                 all_cycle = all_cycle && (state[p] >= 0 || state[p] == kDone);
             }
             s += n;
-            // An orbit that has come back to the value it had a chunk before (as it will from then on) leaves its sums as they
+            // An orbit that has come back to the value it had a chunk before (as it will from then on) keeps its sums as they
             // are there, and the whole chunks that are left are added up from one turn of its cycle: a pixel's bits are its own,
             // whichever others are in its warp, which walks on until all its orbits have, or to the last whole chunk's end.
-            // Cycles walked in full / this: 4096^2 of "AABAB" 200 + 2000 fp32 4.77 / 3.27 ms, fp64 8.37 / 5.65, on the exact orbit
-            // 10.4 / 7.02; 2731 x 1537 of "ABB" 150 + 1500 over [2,4]^2, fp64: 1.61 / 0.91.
+            // Cycles walked in full / this: 4096^2 of "AABAB" 200 + 2000 fp32 4.76 / 3.20 ms, fp64 8.37 / 5.59, on the exact orbit
+            // 10.3 / 6.92; 2731 x 1537 of "ABB" 150 + 1500 over [2,4]^2, fp64: 1.61 / 0.90.
             if (s > whole || (s < whole && !__all_sync(0xFFFFFFFFu, all_cycle))) continue;
 #pragma unroll
             for (int p = 0; p < P; ++p) {
@@ -672,7 +676,8 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                 int exponent;
                 extra[p] = __dadd_rn(extra[p], fast_cycle<FL, KG, ACC_PATS>(kSign * x[p], rA[p], rB[p], rC[p], sel, wrap, s, unit, chunk,
                                                                              q, &exponent));
-                esum[p] += exponent;
+                prod[p] = kept_prod[p][threadIdx.x];
+                esum[p] = kept_esum[p][threadIdx.x] + exponent;
                 valid[p] += q * chunk;
                 if constexpr (FL::same_orbit) {
                     nuse[p][0] += q * cuse[0];
