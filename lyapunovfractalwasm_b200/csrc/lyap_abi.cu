@@ -209,9 +209,9 @@ int launch_lambda(lyap_ctx* c, int mode, lyap::LambdaArgs& a, double* d64, float
     a.cycle_steps = a.queue ? ctx_cycle_steps(c) : nullptr;   // a graph may outlive the context: nothing of the context's goes in
     cudaError_t e;
     if (mode == LYAP_MODE_EXACT) e = lyap::launch_lambda_exact(a, d64, d32, steps, c->sm_count, c->stream);
-    else if (mode == LYAP_MODE_FAST_FP64) e = lyap::launch_lambda_fast64(a, d64, d32, steps, c->sm_count, c->stream);
-    else if (mode == LYAP_MODE_FAST_FP64_ORBIT) e = lyap::launch_lambda_orbit64(a, d64, d32, steps, c->sm_count, c->stream);
-    else e = lyap::launch_lambda_fast32(a, d64, d32, steps, c->sm_count, c->stream);
+    else if (mode == LYAP_MODE_FAST_FP64) e = lyap::launch_lambda_fast64(a, d64, d32, steps, c->stream);
+    else if (mode == LYAP_MODE_FAST_FP64_ORBIT) e = lyap::launch_lambda_orbit64(a, d64, d32, steps, c->stream);
+    else e = lyap::launch_lambda_fast32(a, d64, d32, steps, c->stream);
     if (e != cudaSuccess) return fail_cuda(e, "lambda kernel launch");
     return LYAP_OK;
 }

@@ -12,12 +12,9 @@ namespace lyap {
 
 cudaError_t launch_lambda_exact(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
                                 int sm_count, cudaStream_t st);
-cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                 int sm_count, cudaStream_t st);
-cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                 int sm_count, cudaStream_t st);
-cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                  int sm_count, cudaStream_t st);
+cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st);
+cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st);
+cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st);
 
 // Instance of a lambda kernel made for the sequence's patterns (lyap_jit.cu); kind: 0 exact, 1 fast fp64, 2 fast fp32, 3 fast fp64 on the exact orbit.
 // *launched == false means "not used, launch the generic kernel".  mode: low two bits say when to compile at run time

@@ -1043,18 +1043,15 @@ static cudaError_t launch_lambda_fast_t(const LambdaArgs& a, double* out64, floa
 // Two pixels a thread, which come into cycles together more often than more do and leave registers for more warps: 2731 x 1537
 // of "ABB" 150 + 1500 over [2,4]^2 in fp64 with 4 / 3 / 2 pixels 1.10 / 0.97 / 0.94 ms, 4096^2 of "AABAB" 200 + 2000 in fp32 with
 // 4 / 2 pixels 3.95 / 3.40.
-cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                 int sm_count, cudaStream_t st) {
+cudaError_t launch_lambda_fast64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st) {
     return launch_lambda_fast_t<FusedF64, 2>(a, out64, out32, steps, st, 1, 2, 128, "k_lambda_fast<FusedF64,2,128> (generic)");
 }
 
-cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                 int sm_count, cudaStream_t st) {
+cudaError_t launch_lambda_fast32(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st) {
     return launch_lambda_fast_t<FusedF32, 2>(a, out64, out32, steps, st, 2, 2, 128, "k_lambda_fast<FusedF32,2,128> (generic)");
 }
 
-cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps,
-                                  int sm_count, cudaStream_t st) {
+cudaError_t launch_lambda_orbit64(const LambdaArgs& a, double* out64, float* out32, unsigned long long* steps, cudaStream_t st) {
     return launch_lambda_fast_t<OrbitF64, 2>(a, out64, out32, steps, st, 3, 2, 128, "k_lambda_fast<OrbitF64,2,128> (generic)");
 }
 
