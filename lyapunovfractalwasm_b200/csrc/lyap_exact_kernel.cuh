@@ -496,8 +496,10 @@ __device__ __forceinline__ void exact_tile(const LambdaArgs& a, long long row, i
             // specialised walk: chunks of REP blocks of CB whole periods (>= 16 steps each), then one block, whole periods, single steps
             // REP = 2 blocks between exit tests measured best (1: more tests and state copies; 3 and more: slower code); three of
             // 16 steps hold cycles of three too.  A warp of small tiles that is alone on its scheduler waits some 250 cycles behind
-            // every chunk: four blocks there (128 x 96 of "AABAB" 100 + 4000 over [3.9,4]^2 126 -> 112 us).
-            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, REP = CB * BS == kStepsPerWord ? 3 : (P == 1 && CB * BS <= 20 ? 4 : 2), CS = CB * BS * REP;
+            // every chunk, but replays all of it when an orbit ends there: 128 x 96 of "AABAB" 100 + 4000 over [3.9,4]^2 in chunks of
+            // two / three / four blocks 126 / 118 / 113 us, 205 x 165 90 + 478 over [0,4]^2 56 / 55 / 73.
+            constexpr int BS = 2 * KG, CB = (kStepsPerWord + BS - 1) / BS, BLOCK = CB * BS;
+            constexpr int REP = BLOCK == kStepsPerWord || (P == 1 && BLOCK <= 20) ? 3 : 2, CS = BLOCK * REP;
             static_assert(CS <= kMaxChunk, "an orbit's fall is replayed on the strength of it");
             const unsigned* sel = a.sel + word0;
             int s = 0;
