@@ -599,9 +599,9 @@ def main():
             "flops_per_step": {"warmup": FLOPS_WARM, "accumulated": FLOPS_ACC} if mode == L.MODE_EXACT else FAST_FLOPS,
             "ms_per_launch": ms_lambda,
             # dram__bytes_read.sum + dram__bytes_write.sum of one launch on the 4096x4096 frame, from the ncu capture summarised
-            # under profiles/ (not re-measured by this run): 1.4 MB read + 76.1 MB written; less than the 134 MB of stores
+            # under profiles/ (not re-measured by this run): 16.4 MB read + 110.9 MB written; less than the 134 MB of stores
             # because the tail is still in L2 at kernel end
-            "traffic": 77.5e6 * rows_all / 4096 if mode == L.MODE_EXACT and not strong else None,
+            "traffic": 127.3e6 * rows_all / 4096 if mode == L.MODE_EXACT and not strong else None,
             "traffic_source": "constant from the committed ncu capture of this kernel on this frame, scaled by rows; not measured live",
             "co_bound": {"pipe": "shared-memory data pipe (the logarithm's two 16-byte table look-ups)", "busy": 0.80,
                          "source": "l1tex__data_pipe_lsu_wavefronts_mem_shared, % of peak, from the committed ncu capture of this "

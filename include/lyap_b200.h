@@ -38,15 +38,19 @@ enum lyap_status {
 
 enum lyap_mode {
     LYAP_MODE_EXACT = 0,       /* fp64, reference operation order, one log per step: bit-exact */
-    LYAP_MODE_FAST_FP64 = 1,   /* fp64 FMA orbit, running product of derivatives, one log per pixel */
-    LYAP_MODE_FAST_FP32 = 2,   /* fp32 orbit and products, integer exponent sum, one log per pixel */
+    LYAP_MODE_FAST_FP64 = 1,   /* fp64 FMA orbit, running product of derivatives; logarithms of that product, of one
+                                  turn of an orbit's cycle and of what was redone step by step, not of every step */
+    LYAP_MODE_FAST_FP32 = 2,   /* the same with an fp32 orbit and running product */
     LYAP_MODE_FAST_FP64_ORBIT = 3  /* the reference's own operations for the orbit and for 1 - 2x (so x, the exits and
                                       the sentinels are the exact mode's), but the factors |1 - 2x| multiplied into a
-                                      running product with one log per pixel, and the factors r added as n_A log r_A +
+                                      running product as in the other fast modes, and the factors r added as n_A log r_A +
                                       n_B log r_B (+ n_C log c): lambda differs from the exact mode's only by the
                                       rounding of that accumulation (below 1e-12) */
 };
-/* The fast modes accept at most 2^24 steps per pixel (warmup + iterations): LYAP_ERR_TOO_LARGE beyond. */
+/* The fast modes accept at most 2^24 steps per pixel (warmup + iterations): LYAP_ERR_TOO_LARGE beyond.  In every mode
+ * a pixel's bits depend on its own parameters only, not on the rows, bands or devices it is launched with; in the fast
+ * modes the last digits of a pixel that had steps redone (an exit, a derivative of zero) also depend on whether the
+ * sequence's instance or the generic kernel ran (lyap_last_kernel). */
 
 enum lyap_palette {            /* web/fractal_renderer.js:207-281; unknown names mean cosmic (:280) */
     LYAP_PALETTE_COSMIC = 0,
@@ -124,8 +128,9 @@ int lyap_copy_to_device(lyap_ctx* ctx, void* dev, const void* host, size_t bytes
 /* FractalComputer::computeFractal (src/lyapunov_fractal.hpp:27-102) for rows [row_begin,row_end).
  * d_lambda: rows*width doubles, or NULL; d_lambda32: same count of floats ((float)lambda), or NULL.
  * d_steps: one uint64 the kernel ADDS executed steps to, or NULL.  An orbit that has come back to an earlier value is
- * not walked any further -- the rest of its sum is added up from one turn of its cycle, to the same bits -- but its
- * steps count all the same: they are the reference's.  lyap_cycle_steps says how many were not walked. */
+ * not walked any further: the rest of its sum is added up from one turn of its cycle -- in exact mode to the bits of
+ * the additions one by one, in the fast modes from the logarithm of the turn's product.  Its steps count all the same:
+ * they are the reference's.  lyap_cycle_steps says how many were not walked. */
 int lyap_lambda_device(lyap_ctx* ctx, const lyap_params* p, double* d_lambda, float* d_lambda32,
                        uint64_t* d_steps);
 
@@ -273,7 +278,8 @@ int lyap_minmax_device_noalloc(const double* d_values, uint64_t n, double* d_min
  * the patterns of "AB", "AABAB", "BBBBBBAAAAAA" (500 warm-up steps), "ABC" with a third parameter and "ABB", else one
  * compiled at run time (NVRTC) once about 2e10 steps of work with the sequence have been asked for.  Environment:
  * LYAP_JIT=0 never compiles at run time, 2 compiles on first use; LYAP_PREBUILT=0 ignores the library's own instances
- * (both 0: the generic kernels, which choose the pattern every two steps).
+ * (both 0: the generic kernels, which choose the pattern every two or four steps).  A process that ends while an
+ * instance is being compiled waits for that (a second or two).
  * lyap_jit_note: why the last attempt to build or use a run-time instance fell back ("" if none did).
  * lyap_last_kernel: which lambda kernel the calling thread's last launch used, and how it was made. */
 const char* lyap_jit_note(void);

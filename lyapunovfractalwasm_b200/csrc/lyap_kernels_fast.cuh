@@ -1,13 +1,16 @@
 // lyap_kernels_fast.cuh -- fast-mode lambda kernels (included by lyap_kernels.cu after lyap_exact_kernel.cuh, and, as
 // text, by the run-time specialiser).
 //
-// Same sequence handling, sentinel and early-exit rules as the exact kernel; a thread owns P pixels.  The arithmetic is rearranged for speed and is NOT bit-compatible with the reference:
+// Same sequence handling, sentinel and early-exit rules as the exact kernel; a thread owns P pixels.  The arithmetic is
+// rearranged for speed and is NOT bit-compatible with the reference:
 //   t = r*x;  deriv = fma(-2,t,r) = r(1-2x);  x' = fma(-t,x,t) = r x (1-x)         (4 fused ops/step)
-// and instead of one log per step the |deriv| are multiplied together; the product's exponent is
-// moved into an integer at least every 32 (fp64) or 20 (fp32) steps, and one log of the remaining mantissa is
-// taken per pixel at the end:  sum log|deriv| = E*ln2 + log(mantissa product).
-// A chunk in which the orbit left (0,1) or a derivative was exactly zero is rolled back and redone
-// step by step with the reference's rules (skip zero terms, stop at the exit, keep the partial sum).
+// and instead of one log per step the |deriv| are multiplied together; the product's exponent is moved into an integer at
+// least every 32 (fp64) or 20 (fp32) steps, and one log of the remaining mantissa is taken at the end:
+// sum log|deriv| = E*ln2 + log(mantissa product).
+// A chunk in which the orbit left (0,1) or a derivative was exactly zero is rolled back and redone step by step with the
+// reference's rules (skip zero terms, stop at the exit, keep the partial sum), in a product of its own.  An orbit that
+// stands where it stood a chunk ago is in a cycle, and the chunks that are left are added up from the product of one turn.
+// What a pixel's sum comes to is decided by its own orbit alone, whichever others are in its warp.
 #pragma once
 
 namespace lyap {
