@@ -436,12 +436,12 @@ __device__ __forceinline__ void fast_word(typename FL::real (&x)[P], typename FL
 constexpr int kLeastChunks = 3;
 
 // q times the sum of the logarithms of the derivatives (same orbit: of the factors |1 - 2x|) over n steps, whole periods, of an
-// orbit that stands at x again after them, none of them zero: one turn of its cycle, in units of whole periods, is walked, from
-// step `first` of a region whose selector words start at `sel` (generic kernel) or from a period's start.  The sum is
-// *exponent * log 2 + the result.
+// orbit that stands at x again after them, none of them zero: one turn of its cycle, in units of whole periods, is walked.  The
+// orbit stands behind a whole chunk, at a period's start, and the generic kernel takes the selectors from the beginning of the
+// region's words (`sel`): behind the last chunk there may be fewer than a turn's.  The sum is *exponent * log 2 + the result.
 template <typename FL, int KG, unsigned long long PATS>
 __device__ __noinline__ double fast_cycle(typename FL::real x, typename FL::real rA, typename FL::real rB, typename FL::real rC,
-                                          const unsigned* sel, int wrap, int first, int unit, int n, int q, int* exponent) {
+                                          const unsigned* sel, int wrap, int unit, int n, int q, int* exponent) {
     using T = typename FL::real;
     const T x0 = x;
     LongProduct<FL> product;
@@ -452,10 +452,10 @@ __device__ __noinline__ double fast_cycle(typename FL::real x, typename FL::real
             len += fast_unit(2 * KG);
         } while (x != x0 && len < n);
     } else {
-        const unsigned head = selectors_from(sel, wrap, first);
+        const unsigned head = sel[0];
         do {
             for (int k = 0; k < unit; k += kStepsPerWord) {
-                unsigned word = k == 0 ? head : selectors_from(sel, wrap, first + k);
+                unsigned word = k == 0 ? head : sel[k / kStepsPerWord % wrap];
                 const int m = min(kStepsPerWord, unit - k);
                 for (int j = 0; j < m; ++j, word >>= 2) {
                     const unsigned code = word & 3u;
@@ -677,8 +677,8 @@ __device__ __forceinline__ void lambda_fast_body(const LambdaArgs& a, double* __
                 if (state[p] < 0) continue;
                 const int q = (whole - state[p]) / chunk;
                 int exponent;
-                extra[p] = __dadd_rn(extra[p], fast_cycle<FL, KG, ACC_PATS>(kSign * x[p], rA[p], rB[p], rC[p], sel, wrap, s, unit, chunk,
-                                                                             q, &exponent));
+                extra[p] = __dadd_rn(extra[p], fast_cycle<FL, KG, ACC_PATS>(kSign * x[p], rA[p], rB[p], rC[p], sel, wrap, unit, chunk, q,
+                                                                             &exponent));
                 prod[p] = kept_prod[p][threadIdx.x];
                 esum[p] = kept_esum[p][threadIdx.x] + exponent;
                 valid[p] += q * chunk;

@@ -250,7 +250,9 @@ def test_fast_modes_on_orbits_that_come_into_cycles(engine, port, kernel_path, p
     it, / ln 2 in the mean) and of a few operations at the end; on the reference's orbit also of the parameters' logarithms, of
     which there are as many as steps, each below log2(4)."""
     kernel_path(path)
-    for sequence, iterations in (("AAB", 1000), ("AAB", 72 * 9), ("AB", 96 * 8 + 95), ("AB" * 18 + "A", 1500)):
+    # the last two have their selectors stored whole, none or a few behind the last whole chunk
+    for sequence, iterations in (("AAB", 1000), ("AAB", 72 * 9), ("AB", 96 * 8 + 95), ("AB" * 18 + "A", 1500),
+                                 ("BBAAAAABAB" * 7, 120 * 5 + 4), ("AB" * 18 + "A", 74 * 7)):
         kw = dict(min_x=2.1, max_x=3.0, min_y=2.2, max_y=3.4, width=size[0], height=size[1], sequence=sequence, iterations=iterations,
                   warmup=33)
         for mode, unit in ((L.MODE_FAST_FP64, 2.0 ** -53), (L.MODE_FAST_FP32, 2.0 ** -24), (L.MODE_FAST_FP64_ORBIT, 2.0 ** -53)):
